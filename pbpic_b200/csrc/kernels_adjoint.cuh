@@ -26,6 +26,7 @@ namespace pbd {
 template <class T>
 struct DiffParams {
   PushParams<T> push;     // constants, geometry and the node grid of step n
+  T* s[5];                // the state: dx dy ux uy uz
   int64_t n;              // particles (pairs in load order: 2k ion, 2k+1 electron)
   int64_t nsheet;         // pairs k < nsheet are sheet particles (weight 1)
   double omega_bg;        // weight of background particles
@@ -54,7 +55,7 @@ __global__ void k_dpush(DiffParams<T> a) {
     const T* g10 = g00 + (long long)(pp.my + 1) * 8;
     const Node6<T> n00 = load_node(g00), n01 = load_node(g00 + 8), n10 = load_node(g10), n11 = load_node(g10 + 8);
     Pushed<T> o;
-    push_one<T, false>(pp, sp, ix, iy, pp.dx[p], pp.dy[p], pp.ux[p], pp.uy[p], pp.uz[p], n00, n01, n10, n11, o);
+    push_one<T, false>(pp, sp, ix, iy, a.s[0][p], a.s[1][p], a.s[2][p], a.s[3][p], a.s[4][p], n00, n01, n10, n11, o);
     const double om = particle_weight(a, p);
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
@@ -73,11 +74,11 @@ __global__ void k_dpush(DiffParams<T> a) {
       }
     }
     pp.cell[p] = o.cw;
-    pp.dx[p] = o.dx;
-    pp.dy[p] = o.dy;
-    pp.ux[p] = o.ux;
-    pp.uy[p] = o.uy;
-    pp.uz[p] = o.uz;
+    a.s[0][p] = o.dx;
+    a.s[1][p] = o.dy;
+    a.s[2][p] = o.ux;
+    a.s[3][p] = o.uy;
+    a.s[4][p] = o.uz;
   }
 }
 
@@ -103,9 +104,9 @@ __global__ void k_dadjoint(DiffParams<T> a) {
     const T* g00 = pp.ng + ((long long)ix * (pp.my + 1) + iy) * 8;
     const T* g10 = g00 + (long long)(pp.my + 1) * 8;
     const Node6<T> n00 = load_node(g00), n01 = load_node(g00 + 8), n10 = load_node(g10), n11 = load_node(g10 + 8);
-    const T px = pp.dx[p], py = pp.dy[p];
+    const T px = a.s[0][p], py = a.s[1][p];
     Pushed<T> o;  // the forward push, for the branch decisions and the deposit terms
-    push_one<T, false>(pp, sp, ix, iy, px, py, pp.ux[p], pp.uy[p], pp.uz[p], n00, n01, n10, n11, o);
+    push_one<T, false>(pp, sp, ix, iy, px, py, a.s[2][p], a.s[3][p], a.s[4][p], n00, n01, n10, n11, o);
     const double om = particle_weight(a, p);
     // ---- forward quantities in double
     const double c0 = (double)(sp ? pp.c0[1] : pp.c0[0]), c1 = (double)(sp ? pp.c1[1] : pp.c1[0]);
@@ -120,7 +121,7 @@ __global__ void k_dadjoint(DiffParams<T> a) {
       E = add3(E, scale3(D3{(double)nodes[k]->ex, (double)nodes[k]->ey, (double)nodes[k]->ez}, W[k]));
       B = add3(B, scale3(D3{(double)nodes[k]->bx, (double)nodes[k]->by, (double)nodes[k]->bz}, W[k]));
     }
-    const D3 u{(double)pp.ux[p], (double)pp.uy[p], (double)pp.uz[p]};
+    const D3 u{(double)a.s[2][p], (double)a.s[3][p], (double)a.s[4][p]};
     const D3 um = add3(u, scale3(E, c1));
     const double gm = sqrt(1.0 + dot3(um, um));
     const double c2 = c0 / gm;

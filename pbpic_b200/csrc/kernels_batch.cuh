@@ -28,6 +28,7 @@ static __global__ void k_batch_begin(const BatchDomain* d, int* counters, int* s
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
     counters[0] = 0;
     counters[1] = 0;
+    counters[3] = 0;
     *step += 1;
   }
 }

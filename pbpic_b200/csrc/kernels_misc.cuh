@@ -7,9 +7,9 @@ namespace pbd {
 
 // Device plasma loader: one thread per (ion, electron) pair, the same
 // generator and arithmetic as the host loader in pic_common.h.
-template <class T>
-__global__ void k_load(pic::LoadParams L, int64_t npairs, int electrons_only, uint32_t* cell, T* dx,
-                       T* dy, T* ux, T* uy, T* uz, int32_t* pid) {
+template <class T, class Arrays>
+__global__ void k_load(pic::LoadParams L, int64_t npairs, int electrons_only, uint32_t* cell, Arrays c,
+                       int32_t* pid) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= npairs) return;
   pic::LoadedParticle pr[2];
@@ -17,11 +17,7 @@ __global__ void k_load(pic::LoadParams L, int64_t npairs, int electrons_only, ui
   for (int s = electrons_only ? 1 : 0; s < 2; ++s) {
     const int64_t o = electrons_only ? k : 2 * k + s;
     cell[o] = cw_make(pr[s].ix, pr[s].iy, s);
-    dx[o] = (T)pr[s].ox;
-    dy[o] = (T)pr[s].oy;
-    ux[o] = (T)pr[s].ux;
-    uy[o] = (T)pr[s].uy;
-    uz[o] = (T)pr[s].uz;
+    put_part(c, o, P5<T>{(T)pr[s].ox, (T)pr[s].oy, (T)pr[s].ux, (T)pr[s].uy, (T)pr[s].uz});
     if (pid) pid[o] = (int32_t)(2 * k + s + 1);
   }
 }
@@ -41,8 +37,8 @@ struct RefRec<double> {
 };
 
 template <class T, class R>
-__global__ void k_aos_in(const RefRec<R>* in, int64_t n, int mx, int my, uint32_t* cell, T* dx, T* dy,
-                         T* ux, T* uy, T* uz, int32_t* pid, int* status) {
+__global__ void k_aos_in(const RefRec<R>* in, int64_t n, int mx, int my, uint32_t* cell, Comps<T> c, int32_t* pid,
+                         int* status) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const RefRec<R> r = in[i];
     int g = r.grid - 1;
@@ -52,11 +48,7 @@ __global__ void k_aos_in(const RefRec<R>* in, int64_t n, int mx, int my, uint32_
     }
     const int ix = g / my, iy = g - (g / my) * my;
     cell[i] = cw_make(ix, iy, r.q < 0 ? 1 : 0);
-    dx[i] = (T)r.dx;
-    dy[i] = (T)r.dy;
-    ux[i] = (T)r.ux;
-    uy[i] = (T)r.uy;
-    uz[i] = (T)r.uz;
+    put_part(c, i, P5<T>{(T)r.dx, (T)r.dy, (T)r.ux, (T)r.uy, (T)r.uz});
     if (pid) pid[i] = r.pid;
   }
 }
@@ -64,17 +56,18 @@ __global__ void k_aos_in(const RefRec<R>* in, int64_t n, int mx, int my, uint32_
 // Record i is array element perm[i] (the sort's permutation, not yet applied to
 // the arrays) or element i (perm null).
 template <class T, class R>
-__global__ void k_aos_out(RefRec<R>* out, int64_t n, int my, const int32_t* perm, const uint32_t* cell, const T* dx,
-                          const T* dy, const T* ux, const T* uy, const T* uz, const int32_t* pid) {
+__global__ void k_aos_out(RefRec<R>* out, int64_t n, int my, const int32_t* perm, const uint32_t* cell,
+                          Comps<T> c, const int32_t* pid) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t e = perm ? (int64_t)perm[i] : i;
     const uint32_t w = cell[e];
     RefRec<R> r;
-    r.dx = (R)dx[e];
-    r.dy = (R)dy[e];
-    r.ux = (R)ux[e];
-    r.uy = (R)uy[e];
-    r.uz = (R)uz[e];
+    const P5<T> p = get_part(c, e);
+    r.dx = (R)p.dx;
+    r.dy = (R)p.dy;
+    r.ux = (R)p.ux;
+    r.uy = (R)p.uy;
+    r.uz = (R)p.uz;
     r.grid = my * cw_ix(w) + cw_iy(w) + 1;
     r.q = cw_sp(w) ? -1 : 1;
     r.pid = pid ? pid[e] : 0;
@@ -86,13 +79,13 @@ __global__ void k_aos_out(RefRec<R>* out, int64_t n, int my, const int32_t* perm
 // Kinetic energy per species of the current particles (pic2d.f90:554-568),
 // one partial pair per block.
 template <class T, bool MIXED>
-__global__ void k_kinetic(int64_t n, const uint32_t* cell, const T* ux, const T* uy, const T* uz, T ms_i,
+__global__ void k_kinetic(int64_t n, const uint32_t* cell, Comps<T> p, T ms_i,
                           double* part) {
   __shared__ double red[32];
   double ke[2] = {0, 0};
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     using A = M<T, MIXED>;
-    const T a = ux[i], b = uy[i], c = uz[i];
+    const T a = p.q[4 * i + 2], b = p.q[4 * i + 3], c = p.z[i];
     const T usq = A::mad(c, c, A::mad(b, b, A::mul(a, a)));
     const T g = A::sqrt(A::mad(c, c, A::mad(b, b, A::mad(a, a, T(1)))));
     const int sp = cw_sp(cell[i]);
@@ -110,13 +103,13 @@ __global__ void k_kinetic(int64_t n, const uint32_t* cell, const T* ux, const T*
 // Charge density of the current positions with the gather's CIC weights
 // (pic2d.f90:948-951), unnormalised, into a double plane of mx x S.
 template <class T>
-__global__ void k_rho(int64_t n, int mx, int my, int S, int ybc, const uint32_t* cell, const T* dx,
-                      const T* dy, double* rho) {
+__global__ void k_rho(int64_t n, int mx, int my, int S, int ybc, const uint32_t* cell, Comps<T> p,
+                      double* rho) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t w = cell[i];
     const int ix = cw_ix(w), iy = cw_iy(w);
     const double q = cw_sp(w) ? -1.0 : 1.0;
-    const double ax = 0.5 + (double)dx[i], ay = 0.5 + (double)dy[i];
+    const double ax = 0.5 + (double)p.q[4 * i], ay = 0.5 + (double)p.q[4 * i + 1];
     const double s1 = ax * ay, s2 = ax - s1, s3 = ay - s1, s4 = 1.0 - s1 - s2 - s3;
     const int ip = ix + 1 == mx ? 0 : ix + 1;
     int jp = iy + 1;
@@ -174,13 +167,13 @@ __global__ void k_flux(int mx, int my, const T* ng, double dx, double* out) {
 // here it is counts[species][k-1] (species 0 electrons, 1 ions) and an
 // energy of exactly 0 counts in bin 1. Block histograms in shared memory.
 template <class T>
-__global__ void k_spectra(int64_t n, const uint32_t* cell, const T* ux, const T* uy, const T* uz, double mime,
+__global__ void k_spectra(int64_t n, const uint32_t* cell, Comps<T> p, double mime,
                           double de_e, double de_i, int nbins, unsigned long long* counts) {
   extern __shared__ unsigned int hs[];  // 2 * nbins
   for (int b = threadIdx.x; b < 2 * nbins; b += blockDim.x) hs[b] = 0u;
   __syncthreads();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double x = ux[i], y = uy[i], z = uz[i];  // explicit rounding: no contraction
+    const double x = p.q[4 * i + 2], y = p.q[4 * i + 3], z = p.z[i];  // explicit rounding: no contraction
     const double g2 = __dadd_rn(__dadd_rn(__dadd_rn(1.0, __dmul_rn(x, x)), __dmul_rn(y, y)), __dmul_rn(z, z));
     const double gama = __dsqrt_rn(g2);
     const int sp = cw_sp(cell[i]) ? 0 : 1;  // 0 electron, 1 ion (j = 1, 2 of the reference)

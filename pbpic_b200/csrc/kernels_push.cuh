@@ -60,7 +60,7 @@ struct PushParams {
   int tile_rows, tiles_per_col, ntiles;
   const int32_t* tile_off;  // [ntiles + 1] particle position ranges of the tiles
   uint32_t* cell;
-  T *dx, *dy, *ux, *uy, *uz;
+  Comps<T> c;
   const T* ng;      // node fields (mx+1) x (my+1) x 8: ex ey ez 0 bx by bz 0
   const T* cg;      // mixed form: per-cell gather records mx x my x 24 (k_cell_records)
   void* jacc;       // 4 planes (jx, jy, jz, rho) of mx x S accumulators
@@ -70,11 +70,12 @@ struct PushParams {
   // arrays above; its result goes to element p of the output arrays.
   const int32_t* src;
   uint32_t* cell_o;
-  T *dx_o, *dy_o, *ux_o, *uy_o, *uz_o;
+  Comps<T> c_o;
   const int32_t* pid_i;  // tracked ids, moved with the particles (null: none)
   int32_t* pid_o;
   T c0[2], c1[2], ms[2], qx[2], qy[2], q[2];  // per species: 0 ion, 1 electron
   T dtcva, idx, idy, cva;
+  int lanes;        // lanes per cell of the cell-by-cell push (kernels_push_cells.cuh); 0: the tile push
   double* ke_part;  // [ntiles][2]: electron, ion kinetic energy of the tile
   int* status;
 };
@@ -138,14 +139,6 @@ __device__ __forceinline__ void load_cell(const float* r, Node6<float>& n00, Nod
   n11 = Node6<float>{e.z, e.w, f.x, f.y, f.z, f.w};
 }
 
-__device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
-  const float4 x = *reinterpret_cast<const float4*>(p);
-  v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-}
-__device__ __forceinline__ void ld4(const double* p, double (&v)[4]) {
-  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
 __device__ __forceinline__ void ld4(const uint32_t* p, uint32_t (&v)[4]) {
   const uint4 x = *reinterpret_cast<const uint4*>(p);
   v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
@@ -973,30 +966,26 @@ __device__ __forceinline__ void push_tile(const PushParams<T>& a, const int t, P
           // (a position outside the tile has entry 0: element 0 is read and its values are not used)
           const int e = sidx[j];
           cw[j] = __ldg(a.cell + e);
-          px[j] = __ldg(a.dx + e);
-          py[j] = __ldg(a.dy + e);
-          pux[j] = __ldg(a.ux + e);
-          puy[j] = __ldg(a.uy + e);
-          puz[j] = __ldg(a.uz + e);
+          const P5<T> v = ldg_part(a.c, e);
+          px[j] = v.dx;
+          py[j] = v.dy;
+          pux[j] = v.ux;
+          puy[j] = v.uy;
+          puz[j] = v.uz;
         }
-      } else if (full) {
-        ld4(a.cell + q, cw);
-        ld4(a.dx + q, px);
-        ld4(a.dy + q, py);
-        ld4(a.ux + q, pux);
-        ld4(a.uy + q, puy);
-        ld4(a.uz + q, puz);
       } else {
+        if (full) ld4(a.cell + q, cw);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int p = q + j;
-          const bool act = p >= pbeg && p < pend;
-          cw[j] = act ? a.cell[p] : 0u;
-          px[j] = act ? a.dx[p] : T(0);
-          py[j] = act ? a.dy[p] : T(0);
-          pux[j] = act ? a.ux[p] : T(0);
-          puy[j] = act ? a.uy[p] : T(0);
-          puz[j] = act ? a.uz[p] : T(0);
+          const bool act = full || (p >= pbeg && p < pend);
+          if (!full) cw[j] = act ? a.cell[p] : 0u;
+          const P5<T> v = act ? get_part(a.c, p) : P5<T>{};
+          px[j] = v.dx;
+          py[j] = v.dy;
+          pux[j] = v.ux;
+          puy[j] = v.uy;
+          puz[j] = v.uz;
         }
       }
 #if PBPIC_PUSH_UNROLL
@@ -1178,26 +1167,21 @@ __device__ __forceinline__ void push_tile(const PushParams<T>& a, const int t, P
         else pke_i += o.ke;
       }
       uint32_t* ocell = GATHER ? a.cell_o : a.cell;
-      T *odx = GATHER ? a.dx_o : a.dx, *ody = GATHER ? a.dy_o : a.dy;
-      T *oux = GATHER ? a.ux_o : a.ux, *ouy = GATHER ? a.uy_o : a.uy, *ouz = GATHER ? a.uz_o : a.uz;
+      const Comps<T>& oc = GATHER ? a.c_o : a.c;
       if (full) {
         st4(ocell + q, cw);
-        st4(odx + q, px);
-        st4(ody + q, py);
-        st4(oux + q, pux);
-        st4(ouy + q, puy);
-        st4(ouz + q, puz);
+        st4(oc.z + q, puz);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          put_quad(oc, q + j, px[j], py[j], pux[j], puy[j]);
+        }
       } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int p = q + j;
           if (p >= pbeg && p < pend) {
             ocell[p] = cw[j];
-            odx[p] = px[j];
-            ody[p] = py[j];
-            oux[p] = pux[j];
-            ouy[p] = puy[j];
-            ouz[p] = puz[j];
+            put_part(oc, p, P5<T>{px[j], py[j], pux[j], puy[j], puz[j]});
           }
         }
       }

@@ -34,18 +34,18 @@ static __global__ void k_band_flags(int64_t n, const uint32_t* cell, int y_lo, i
 // Particles with a flag to out[pos[i]] as reference records of the global
 // grid: grid = my_global * ix + (iy + row_offset) + 1, q = +1 ion / -1 electron.
 template <class T, class R>
-__global__ void k_band_out(int64_t n, const uint32_t* cell, const T* dx, const T* dy, const T* ux, const T* uy,
-                           const T* uz, const int32_t* pid, const int32_t* pos, int my_global, int row_offset,
+__global__ void k_band_out(int64_t n, const uint32_t* cell, Comps<T> c, const int32_t* pid, const int32_t* pos, int my_global, int row_offset,
                            RefRec<R>* out) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     if (pos[i + 1] == pos[i]) continue;  // not in the band
     const uint32_t w = cell[i];
     RefRec<R> r;
-    r.dx = (R)dx[i];
-    r.dy = (R)dy[i];
-    r.ux = (R)ux[i];
-    r.uy = (R)uy[i];
-    r.uz = (R)uz[i];
+    const P5<T> p = get_part(c, i);
+    r.dx = (R)p.dx;
+    r.dy = (R)p.dy;
+    r.ux = (R)p.ux;
+    r.uy = (R)p.uy;
+    r.uz = (R)p.uz;
     r.grid = my_global * cw_ix(w) + cw_iy(w) + row_offset + 1;
     r.q = cw_sp(w) ? -1 : 1;
     r.pid = pid ? pid[i] : 0;
@@ -55,18 +55,13 @@ __global__ void k_band_out(int64_t n, const uint32_t* cell, const T* dx, const T
 
 // Stable compaction of the flagged particles into the other buffer.
 template <class T>
-__global__ void k_band_keep(int64_t n, const int32_t* pos, const uint32_t* ci, const T* dxi, const T* dyi,
-                            const T* uxi, const T* uyi, const T* uzi, const int32_t* pidi, uint32_t* co, T* dxo,
-                            T* dyo, T* uxo, T* uyo, T* uzo, int32_t* pido) {
+__global__ void k_band_keep(int64_t n, const int32_t* pos, const uint32_t* ci, Comps<T> in, const int32_t* pidi, uint32_t* co,
+                            Comps<T> out, int32_t* pido) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     if (pos[i + 1] == pos[i]) continue;
     const int64_t d = pos[i];
     co[d] = ci[i];
-    dxo[d] = dxi[i];
-    dyo[d] = dyi[i];
-    uxo[d] = uxi[i];
-    uyo[d] = uyi[i];
-    uzo[d] = uzi[i];
+    put_part(out, d, get_part(in, i));
     if (pido) pido[d] = pidi[i];
   }
 }
@@ -77,7 +72,7 @@ __global__ void k_band_keep(int64_t n, const int32_t* pos, const uint32_t* ci, c
 // otherwise, so that the count stays consistent).
 template <class T, class R>
 __global__ void k_band_in(const RefRec<R>* in, int64_t n, int my_global, int row_offset, int mx, int my, int64_t base,
-                          uint32_t* cell, T* dx, T* dy, T* ux, T* uy, T* uz, int32_t* pid, int* status) {
+                          uint32_t* cell, Comps<T> c, int32_t* pid, int* status) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const RefRec<R> r = in[i];
     const int g = r.grid - 1;
@@ -87,11 +82,7 @@ __global__ void k_band_in(const RefRec<R>* in, int64_t n, int my_global, int row
     const int64_t d = base + i;
     if (!ok) atomicOr(status, 8);
     cell[d] = ok ? cw_make(ix, iy, r.q < 0 ? 1 : 0) : cw_make(0, 0, 1);
-    dx[d] = ok ? (T)r.dx : T(0);
-    dy[d] = ok ? (T)r.dy : T(0);
-    ux[d] = ok ? (T)r.ux : T(0);
-    uy[d] = ok ? (T)r.uy : T(0);
-    uz[d] = ok ? (T)r.uz : T(0);
+    put_part(c, d, ok ? P5<T>{(T)r.dx, (T)r.dy, (T)r.ux, (T)r.uy, (T)r.uz} : P5<T>{});
     if (pid) pid[d] = r.pid;
   }
 }
@@ -126,7 +117,7 @@ __global__ void k_rows_set(Planes6<T> p, int mx, int S, int j0, int nrows, const
 
 // Kinetic energy of the particles in rows [y_lo, y_hi), as k_kinetic.
 template <class T, bool MIXED>
-__global__ void k_kinetic_rows(int64_t n, const uint32_t* cell, const T* ux, const T* uy, const T* uz, T ms_i,
+__global__ void k_kinetic_rows(int64_t n, const uint32_t* cell, Comps<T> p, T ms_i,
                                int y_lo, int y_hi, double* part) {
   __shared__ double red[32];
   double ke[2] = {0, 0};
@@ -135,7 +126,7 @@ __global__ void k_kinetic_rows(int64_t n, const uint32_t* cell, const T* ux, con
     const int iy = cw_iy(w);
     if (iy < y_lo || iy >= y_hi) continue;
     using A = M<T, MIXED>;
-    const T a = ux[i], b = uy[i], c = uz[i];
+    const T a = p.q[4 * i + 2], b = p.q[4 * i + 3], c = p.z[i];
     const T usq = A::mad(c, c, A::mad(b, b, A::mul(a, a)));
     const T g = A::sqrt(A::mad(c, c, A::mad(b, b, A::mad(a, a, T(1)))));
     const int sp = cw_sp(w);
@@ -221,8 +212,7 @@ __device__ __forceinline__ void store_record(RefRec<double>* p, const RefRec<dou
 // block per column (grid-stride over the columns).
 template <class T, class R>
 __global__ void k_band_out_sorted(const int32_t* colstart, const int32_t* off, int mx, int my, int y_lo,
-                                  const uint32_t* cell, const T* dx, const T* dy, const T* ux, const T* uy,
-                                  const T* uz, const int32_t* pid, int my_global, int row_offset, RefRec<R>* out,
+                                  const uint32_t* cell, Comps<T> c, const int32_t* pid, int my_global, int row_offset, RefRec<R>* out,
                                   const int32_t* perm, bool al16) {
   for (int ix = blockIdx.x; ix < mx; ix += gridDim.x) {
     const int64_t k0 = colstart[ix], k1 = colstart[ix + 1];
@@ -232,11 +222,12 @@ __global__ void k_band_out_sorted(const int32_t* colstart, const int32_t* off, i
       const int64_t i = perm ? (int64_t)perm[j] : j;
       const uint32_t w = cell[i];
       RefRec<R> r;
-      r.dx = (R)dx[i];
-      r.dy = (R)dy[i];
-      r.ux = (R)ux[i];
-      r.uy = (R)uy[i];
-      r.uz = (R)uz[i];
+      const P5<T> p = get_part(c, i);
+      r.dx = (R)p.dx;
+      r.dy = (R)p.dy;
+      r.ux = (R)p.ux;
+      r.uy = (R)p.uy;
+      r.uz = (R)p.uz;
       r.grid = my_global * cw_ix(w) + cw_iy(w) + row_offset + 1;
       r.q = cw_sp(w) ? -1 : 1;
       r.pid = pid ? pid[i] : 0;
@@ -289,9 +280,8 @@ struct ReplaceSrc {
 
 template <class T, class R>
 __global__ void k_band_assemble(int64_t total, ReplaceSrc s, const RefRec<R>* bot, const RefRec<R>* top,
-                                const uint32_t* ci, const T* dxi, const T* dyi, const T* uxi, const T* uyi,
-                                const T* uzi, const int32_t* pidi, uint32_t* co, T* dxo, T* dyo, T* uxo, T* uyo,
-                                T* uzo, int32_t* pido, int* status, const int32_t* perm) {
+                                const uint32_t* ci, Comps<T> in, const int32_t* pidi, uint32_t* co, Comps<T> out,
+                                int32_t* pido, int* status, const int32_t* perm) {
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
     const int ix = column_of(s.outstart, s.mx, k);
     int64_t r = k - s.outstart[ix];
@@ -300,11 +290,7 @@ __global__ void k_band_assemble(int64_t total, ReplaceSrc s, const RefRec<R>* bo
       const int64_t j = (int64_t)s.off[(int64_t)ix * s.my + s.y_lo] + (r - nb);
       const int64_t i = perm ? (int64_t)perm[j] : j;
       co[k] = ci[i];
-      dxo[k] = dxi[i];
-      dyo[k] = dyi[i];
-      uxo[k] = uxi[i];
-      uyo[k] = uyi[i];
-      uzo[k] = uzi[i];
+      put_part(out, k, get_part(in, i));
       if (pido) pido[k] = pidi[i];
       continue;
     }
@@ -316,11 +302,7 @@ __global__ void k_band_assemble(int64_t total, ReplaceSrc s, const RefRec<R>* bo
     const bool ok = gx == ix && iy >= 0 && iy < s.my && (rec.q == 1 || rec.q == -1);
     if (!ok) atomicOr(status, 8);
     co[k] = ok ? cw_make(ix, iy, rec.q < 0 ? 1 : 0) : cw_make(ix, s.y_lo, 1);
-    dxo[k] = ok ? (T)rec.dx : T(0);
-    dyo[k] = ok ? (T)rec.dy : T(0);
-    uxo[k] = ok ? (T)rec.ux : T(0);
-    uyo[k] = ok ? (T)rec.uy : T(0);
-    uzo[k] = ok ? (T)rec.uz : T(0);
+    put_part(out, k, ok ? P5<T>{(T)rec.dx, (T)rec.dy, (T)rec.ux, (T)rec.uy, (T)rec.uz} : P5<T>{});
     if (pido) pido[k] = rec.pid;
   }
 }
@@ -333,7 +315,7 @@ __global__ void k_band_assemble(int64_t total, ReplaceSrc s, const RefRec<R>* bo
 // next push reads through. The own particles stay where they are.
 template <class T, class R>
 __global__ void k_band_to_soa(int64_t nb, int64_t nt, ReplaceSrc s, const RefRec<R>* bot, const RefRec<R>* top,
-                              int64_t base, uint32_t* co, T* dxo, T* dyo, T* uxo, T* uyo, T* uzo, int32_t* pido,
+                              int64_t base, uint32_t* co, Comps<T> out, int32_t* pido,
                               int* status) {
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nb + nt; k += (int64_t)gridDim.x * blockDim.x) {
     const bool lower = k < nb;
@@ -345,11 +327,7 @@ __global__ void k_band_to_soa(int64_t nb, int64_t nt, ReplaceSrc s, const RefRec
     if (!ok) atomicOr(status, 8);
     const int64_t e = base + k;
     co[e] = ok ? cw_make(gx, iy, rec.q < 0 ? 1 : 0) : cw_make(gx >= 0 && gx < s.mx ? gx : 0, s.y_lo, 1);
-    dxo[e] = ok ? (T)rec.dx : T(0);
-    dyo[e] = ok ? (T)rec.dy : T(0);
-    uxo[e] = ok ? (T)rec.ux : T(0);
-    uyo[e] = ok ? (T)rec.uy : T(0);
-    uzo[e] = ok ? (T)rec.uz : T(0);
+    put_part(out, e, ok ? P5<T>{(T)rec.dx, (T)rec.dy, (T)rec.ux, (T)rec.uy, (T)rec.uz} : P5<T>{});
     if (pido) pido[e] = rec.pid;
   }
 }

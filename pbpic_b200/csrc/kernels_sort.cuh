@@ -138,19 +138,13 @@ static __global__ void k_runs_ok(const int32_t* nruns, int64_t ncells, int* flag
 
 template <class T>
 __global__ void k_run_scatter(int64_t n, int my, const int32_t* off, const int32_t* runstart, const uint32_t* ci,
-                              const T* dxi, const T* dyi, const T* uxi, const T* uyi, const T* uzi,
-                              const int32_t* pidi, uint32_t* co, T* dxo, T* dyo, T* uxo, T* uyo, T* uzo,
-                              int32_t* pido) {
+                              Comps<T> in, const int32_t* pidi, uint32_t* co, Comps<T> out, int32_t* pido) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t w = ci[i];
     const int key = cw_ix(w) * my + cw_iy(w);
     const int64_t d = (int64_t)off[key] + (i - runstart[key]);
     co[d] = w;
-    dxo[d] = dxi[i];
-    dyo[d] = dyi[i];
-    uxo[d] = uxi[i];
-    uyo[d] = uyi[i];
-    uzo[d] = uzi[i];
+    put_part(out, d, get_part(in, i));
     if (pido) pido[d] = pidi[i];
   }
 }
@@ -246,17 +240,12 @@ static __global__ void __launch_bounds__(RB) k_radix_down(const int32_t* kin, co
 
 // ----------------------------------------------------------------- gather
 template <class T>
-__global__ void k_gather(const int32_t* perm, int64_t n, const uint32_t* ci, const T* dxi, const T* dyi,
-                         const T* uxi, const T* uyi, const T* uzi, const int32_t* pidi, uint32_t* co,
-                         T* dxo, T* dyo, T* uxo, T* uyo, T* uzo, int32_t* pido) {
+__global__ void k_gather(const int32_t* perm, int64_t n, const uint32_t* ci,
+                              Comps<T> in, const int32_t* pidi, uint32_t* co, Comps<T> out, int32_t* pido) {
   for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
     const int32_t s = perm[j];
     co[j] = ci[s];
-    dxo[j] = dxi[s];
-    dyo[j] = dyi[s];
-    uxo[j] = uxi[s];
-    uyo[j] = uyi[s];
-    uzo[j] = uzi[s];
+    put_part(out, j, get_part(in, s));
     if (pido) pido[j] = pidi[s];
   }
 }

@@ -20,6 +20,7 @@
 #include "kernels_field.cuh"
 #include "kernels_misc.cuh"
 #include "kernels_push.cuh"
+#include "kernels_push_cells.cuh"
 #include "kernels_slab.cuh"
 #include "kernels_sort.cuh"
 #include "h5_writer.h"
@@ -143,7 +144,8 @@ struct pbpic_handle {
   int S = 0, ncells = 0, TY = 0, tpc = 0, ntiles = 0;
   int64_t n = 0, cap = 0;
   uint32_t* cell[2] = {nullptr, nullptr};
-  void* comp[2][5] = {{nullptr}};
+  void* quad[2] = {nullptr, nullptr};  // dx dy ux uy of each particle
+  void* uz[2] = {nullptr, nullptr};
   int32_t* pid[2] = {nullptr, nullptr};
   int cur = 0;
   void* f[6] = {nullptr};
@@ -285,8 +287,23 @@ int ensure_hist(pbpic_handle* h, int rows) {
 }
 
 template <class T>
-T* P(pbpic_handle* h, int buf, int c) {
-  return (T*)h->comp[buf][c];
+Comps<T> C(pbpic_handle* h, int buf) {
+  return Comps<T>{(T*)h->quad[buf], (T*)h->uz[buf]};
+}
+
+// Lanes per cell of the push cell by cell (kernels_push_cells.cuh: sorted input, no compat
+// switch, not the exact order), 0 for the tile push. By the domain's mean particles
+// per cell, uniform plasma on 512x256 cells, us per step.
+// Mixed, tile push / 16 lanes / 32 lanes: 8: 168 / 178 / 206; 16: 186 / 189 / 220;
+// 24: 207 / 192 / 220; 64: 307 / 253 / 284; 128: 484 / 343 / 363; 200: 664 / 468 / 472
+// (a Harris sheet of 200: 16 lanes 518, 32 lanes 505).
+// Plain, tile push / 32 lanes (16 lanes never better): 16: 244 / 293; 24: 286 / 304;
+// 64: 501 / 399; 128: 826 / 556; 180: 1097 / 685.
+int cells_lanes(const pbpic_handle* h) {
+  if (h->cfg.compat != 0 || (!h->mixed && (h->cfg.options & PBPIC_OPT_EXACT_FP64))) return 0;
+  const double per_cell = (double)h->n / (double)h->ncells;
+  if (!h->mixed) return per_cell < 30.0 ? 0 : 32;
+  return per_cell < 16.0 ? 0 : (per_cell < 180.0 ? 16 : 32);
 }
 
 // ------------------------------------------------------------- constants
@@ -305,11 +322,7 @@ PushParams<T> push_params(pbpic_handle* h) {
   p.tile_off = h->tile_off;
   const int b = h->cur;
   p.cell = h->cell[b];
-  p.dx = P<T>(h, b, 0);
-  p.dy = P<T>(h, b, 1);
-  p.ux = P<T>(h, b, 2);
-  p.uy = P<T>(h, b, 3);
-  p.uz = P<T>(h, b, 4);
+  p.c = C<T>(h, b);
   p.ng = (const T*)h->ng;
   p.cg = (const T*)h->cg;
   p.jacc = h->jacc;
@@ -317,7 +330,7 @@ PushParams<T> push_params(pbpic_handle* h) {
   p.cell_off = h->off;
   p.src = nullptr;
   p.cell_o = nullptr;
-  p.dx_o = p.dy_o = p.ux_o = p.uy_o = p.uz_o = nullptr;
+  p.c_o = Comps<T>{nullptr, nullptr};
   p.pid_i = nullptr;
   p.pid_o = nullptr;
   const T dt = (T)c.dt, mime = (T)c.mime, cva = (T)c.cva, dx = (T)c.dx, dy = (T)c.dy;
@@ -335,6 +348,7 @@ PushParams<T> push_params(pbpic_handle* h) {
   p.idx = T(1) / dx;   // pic2d.f90:16
   p.idy = T(1) / dy;
   p.cva = cva;
+  p.lanes = cells_lanes(h);
   p.ke_part = h->ke_part;
   p.status = h->status;
   return p;
@@ -417,8 +431,7 @@ template <class T, bool MIXED>
 int kinetic_row(pbpic_handle* h, int row) {
   TRY(ensure_hist(h, row + 1));
   const int b = h->cur;
-  k_kinetic<T, MIXED><<<h->nke, 256, 0, h->stream>>>(h->n, h->cell[b], P<T>(h, b, 2), P<T>(h, b, 3),
-                                                      P<T>(h, b, 4), (T)h->cfg.mime, h->ke_part);
+  k_kinetic<T, MIXED><<<h->nke, 256, 0, h->stream>>>(h->n, h->cell[b], C<T>(h, b), (T)h->cfg.mime, h->ke_part);
   CKLAUNCH("k_kinetic");
   k_energy_row<<<1, 256, 0, h->stream>>>(h->ke_part, h->nke, nullptr, 0, 0, 0, h->hist + (size_t)row * 4);
   CKLAUNCH("k_energy_row");
@@ -432,10 +445,8 @@ int materialize_t(pbpic_handle* h) {
   const int64_t n = h->n;
   const int b = h->cur, o = 1 - b;
   if (n > 0) {
-    k_gather<T><<<grid_for(n, 256), 256, 0, h->stream>>>(h->perm, n, h->cell[b], P<T>(h, b, 0), P<T>(h, b, 1),
-                                                          P<T>(h, b, 2), P<T>(h, b, 3), P<T>(h, b, 4), h->pid[b],
-                                                          h->cell[o], P<T>(h, o, 0), P<T>(h, o, 1), P<T>(h, o, 2),
-                                                          P<T>(h, o, 3), P<T>(h, o, 4), h->pid[o]);
+    k_gather<T><<<grid_for(n, 256), 256, 0, h->stream>>>(h->perm, n, h->cell[b], C<T>(h, b), h->pid[b],
+                                                          h->cell[o], C<T>(h, o), h->pid[o]);
     CKLAUNCH("k_gather");
     h->cur = o;
   }
@@ -491,10 +502,8 @@ int do_sort(pbpic_handle* h) {
     CK(cudaMemcpyAsync(&many, flag, 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     if (!many) {
-      k_run_scatter<T><<<grid_for(n, 256), 256, 0, s>>>(n, h->cfg.my, h->off, runstart, h->cell[b], P<T>(h, b, 0),
-                                                        P<T>(h, b, 1), P<T>(h, b, 2), P<T>(h, b, 3), P<T>(h, b, 4),
-                                                        h->pid[b], h->cell[o], P<T>(h, o, 0), P<T>(h, o, 1),
-                                                        P<T>(h, o, 2), P<T>(h, o, 3), P<T>(h, o, 4), h->pid[o]);
+      k_run_scatter<T><<<grid_for(n, 256), 256, 0, s>>>(n, h->cfg.my, h->off, runstart, h->cell[b], C<T>(h, b),
+                                                        h->pid[b], h->cell[o], C<T>(h, o), h->pid[o]);
       CKLAUNCH("k_run_scatter");
       h->cur = o;
       runs = true;
@@ -504,9 +513,7 @@ int do_sort(pbpic_handle* h) {
     int32_t* perm = nullptr;
     TRY(radix_sort(s, n, h->ncells, h->keys[0], h->keys[1], h->vals[0], h->vals[1], h->rhist, h->scan_scratch,
                    &perm));
-    k_gather<T><<<grid_for(n, 256), 256, 0, s>>>(perm, n, h->cell[b], P<T>(h, b, 0), P<T>(h, b, 1), P<T>(h, b, 2),
-                                                  P<T>(h, b, 3), P<T>(h, b, 4), h->pid[b], h->cell[o], P<T>(h, o, 0),
-                                                  P<T>(h, o, 1), P<T>(h, o, 2), P<T>(h, o, 3), P<T>(h, o, 4),
+    k_gather<T><<<grid_for(n, 256), 256, 0, s>>>(perm, n, h->cell[b], C<T>(h, b), h->pid[b], h->cell[o], C<T>(h, o),
                                                   h->pid[o]);
     CKLAUNCH("k_gather");
     h->cur = o;
@@ -516,6 +523,15 @@ int do_sort(pbpic_handle* h) {
   CKLAUNCH("k_tile_off");
   h->sorted = true;
   h->hist_valid = false;
+  return PBPIC_OK;
+}
+
+template <class T, bool GATHER>
+int launch_push_cells(pbpic_handle* h, const PushParams<T>& p) {
+  const size_t smem = cells_smem_bytes(h->TY, sizeof(T) == 4);
+  auto run = [&](auto kernel) { kernel<<<h->ntiles, PC_THREADS, smem, h->stream>>>(p); };
+  if (sizeof(T) == 8 || p.lanes == 32) p.pid_o ? run(k_push_cells<T, 32, GATHER, GATHER>) : run(k_push_cells<T, 32, GATHER, false>);
+  else if constexpr (sizeof(T) == 4) p.pid_o ? run(k_push_cells<T, 16, GATHER, GATHER>) : run(k_push_cells<T, 16, GATHER, false>);
   return PBPIC_OK;
 }
 
@@ -536,25 +552,24 @@ int do_push(pbpic_handle* h) {
   const int nt = PushThreads<T>::value;
   // the compat instances also carry the plain form's exact-order arithmetic
   const bool compat = h->cfg.compat != 0 || (!MIXED && (h->cfg.options & PBPIC_OPT_EXACT_FP64));
+  const bool cells = hist && p.lanes > 0;
   if (h->lazy) {  // read through the sort's permutation, write in cell order to the other buffer
     if (!hist) return fail(PBPIC_ESTATE, "k_push: a permuted input needs the sort's tables");
     const int o = 1 - h->cur;
     p.src = h->perm;
     p.cell_o = h->cell[o];
-    p.dx_o = P<T>(h, o, 0);
-    p.dy_o = P<T>(h, o, 1);
-    p.ux_o = P<T>(h, o, 2);
-    p.uy_o = P<T>(h, o, 3);
-    p.uz_o = P<T>(h, o, 4);
+    p.c_o = C<T>(h, o);
     p.pid_i = h->pid[h->cur];
     p.pid_o = h->pid[o];
-    if (!compat) k_push<T, MIXED, true, false, true><<<h->ntiles, nt, smem, s>>>(p);
+    if (cells) TRY((launch_push_cells<T, true>(h, p)));
+    else if (!compat) k_push<T, MIXED, true, false, true><<<h->ntiles, nt, smem, s>>>(p);
     else k_push<T, MIXED, true, true, true><<<h->ntiles, nt, smem, s>>>(p);
     CKLAUNCH("k_push");
     h->cur = o;
     h->lazy = false;
   } else {
-    if (hist && !compat) k_push<T, MIXED, true, false><<<h->ntiles, nt, smem, s>>>(p);
+    if (cells) TRY((launch_push_cells<T, false>(h, p)));
+    else if (hist && !compat) k_push<T, MIXED, true, false><<<h->ntiles, nt, smem, s>>>(p);
     else if (hist) k_push<T, MIXED, true, true><<<h->ntiles, nt, smem, s>>>(p);
     else if (!compat) k_push<T, MIXED, false, false><<<h->ntiles, nt, smem, s>>>(p);
     else k_push<T, MIXED, false, true><<<h->ntiles, nt, smem, s>>>(p);
@@ -780,8 +795,7 @@ int do_load_aos(pbpic_handle* h, const RefRec<R>* host, int64_t n) {
     CK(cudaMemcpyAsync(h->staging, host, (size_t)n * sizeof(RefRec<R>), cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
     k_aos_in<T, R><<<grid_for(n, 256), 256, 0, h->stream>>>((const RefRec<R>*)h->staging, n, h->cfg.mx, h->cfg.my,
-                                                              h->cell[b], P<T>(h, b, 0), P<T>(h, b, 1),
-                                                              P<T>(h, b, 2), P<T>(h, b, 3), P<T>(h, b, 4),
+                                                              h->cell[b], C<T>(h, b),
                                                               h->pid[b], h->status);
     CKLAUNCH("k_aos_in");
     int st = 0;
@@ -805,8 +819,7 @@ int do_store_aos(pbpic_handle* h, RefRec<R>* host, int64_t cap, int64_t* nout) {
   TRY(ensure_staging(h, (size_t)n * sizeof(RefRec<R>)));
   k_aos_out<T, R><<<grid_for(n, 256), 256, 0, h->stream>>>((RefRec<R>*)h->staging, n, h->cfg.my,
                                                              h->lazy ? h->perm : nullptr, h->cell[b],
-                                                             P<T>(h, b, 0), P<T>(h, b, 1), P<T>(h, b, 2),
-                                                             P<T>(h, b, 3), P<T>(h, b, 4), h->pid[b]);
+                                                             C<T>(h, b), h->pid[b]);
   CKLAUNCH("k_aos_out");
   CK(cudaMemcpyAsync(host, h->staging, (size_t)n * sizeof(RefRec<R>), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -877,8 +890,7 @@ int do_init_plasma(pbpic_handle* h, const pbpic_loader* ld) {
   const int b = h->cur;
   if (L.npairs > 0) {
     k_load<T><<<(unsigned)((L.npairs + 255) / 256), 256, 0, h->stream>>>(
-        L, L.npairs, ld->immobile_ions, h->cell[b], P<T>(h, b, 0), P<T>(h, b, 1), P<T>(h, b, 2), P<T>(h, b, 3),
-        P<T>(h, b, 4), h->pid[b]);
+        L, L.npairs, ld->immobile_ions, h->cell[b], C<T>(h, b), h->pid[b]);
     CKLAUNCH("k_load");
   }
   h->n = n;
@@ -921,7 +933,7 @@ int do_gauss(pbpic_handle* h, double* out, int jlo, int jhi) {
   const int b = h->cur;
   if (h->n > 0) {
     k_rho<T><<<grid_for(h->n, 256), 256, 0, s>>>(h->n, h->cfg.mx, h->cfg.my, h->S, h->cfg.ybc, h->cell[b],
-                                                  P<T>(h, b, 0), P<T>(h, b, 1), h->rho);
+                                                  C<T>(h, b), h->rho);
     CKLAUNCH("k_rho");
   }
   const pbpic_config& c = h->cfg;
@@ -1012,7 +1024,8 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
   for (int b = 0; b < 2; ++b) {
     // particle arrays carry 16 elements of padding: bulk copies read whole 16-byte units
     A(&h->cell[b], (capn + 16) * 4);
-    for (int k = 0; k < 5; ++k) A(&h->comp[b][k], (capn + 16) * h->tsz);
+    A(&h->quad[b], (capn + 16) * 4 * h->tsz);
+    A(&h->uz[b], (capn + 16) * h->tsz);
     if (c.track_pid) A(&h->pid[b], (capn + 16) * 4);
     A(&h->keys[b], capn * 4);
     A(&h->vals[b], capn * 4);
@@ -1228,12 +1241,10 @@ int pbpic_energy_spectra(pbpic_handle* h, double de_electron, double de_ion, int
   if (h->n > 0) {
     const int g = grid_for(h->n, 256, 148 * 4);
     if (h->mixed)
-      k_spectra<float><<<g, 256, (size_t)2 * nbins * 4, s>>>(h->n, h->cell[b], P<float>(h, b, 2), P<float>(h, b, 3),
-                                                            P<float>(h, b, 4), h->cfg.mime, de_electron, de_ion, nbins,
+      k_spectra<float><<<g, 256, (size_t)2 * nbins * 4, s>>>(h->n, h->cell[b], C<float>(h, b), h->cfg.mime, de_electron, de_ion, nbins,
                                                             (unsigned long long*)h->staging);
     else
-      k_spectra<double><<<g, 256, (size_t)2 * nbins * 4, s>>>(h->n, h->cell[b], P<double>(h, b, 2),
-                                                             P<double>(h, b, 3), P<double>(h, b, 4), h->cfg.mime,
+      k_spectra<double><<<g, 256, (size_t)2 * nbins * 4, s>>>(h->n, h->cell[b], C<double>(h, b), h->cfg.mime,
                                                              de_electron, de_ion, nbins,
                                                              (unsigned long long*)h->staging);
     CKLAUNCH("k_spectra");
@@ -1538,9 +1549,11 @@ struct pbpic_batch {
   BatchDomain* d_dom = nullptr;
   EnergyRow* d_erow = nullptr;
   int2* d_tiles = nullptr;
-  int* d_counters = nullptr;  // [0] push, [1] scatter, [2] step index
+  int* d_counters = nullptr;  // [0] tile push, [1] scatter, [2] step index, [3] push cell by cell
   int ntiles = 0, push_blocks = 0, scatter_blocks = 0;
-  size_t push_smem = 0;
+  int ncells_tiles = 0, cells_blocks = 0;  // the table's first tiles: those pushed cell by cell
+  bool track = false;                      // some domain carries particle ids
+  size_t push_smem = 0, cells_smem = 0;
   int gx_zero = 1, gx_cells = 1, gx_bins = 1, gx_tiles = 1, gx_field = 1, gx_nodes = 1;
 };
 
@@ -1625,9 +1638,11 @@ int batch_layout(pbpic_batch* b) {
   struct Item {
     double cost;
     int d, t;
+    bool cells;
   };
   std::vector<Item> items;
-  size_t smem = 0;
+  size_t smem = 0, csmem = 0;
+  bool track = false;
   int64_t maxcells = 1, maxbins = 1, maxtiles = 1, maxfield = 1, maxacc = 1;
   int maxnfe = 1;
   for (int d = 0; d < D; ++d) {
@@ -1636,9 +1651,11 @@ int batch_layout(pbpic_batch* b) {
     for (int t = 0; t < h->ntiles; ++t) {
       const int y0 = (t % h->tpc) * h->TY;
       const int rows = std::min(h->TY, h->cfg.my - y0);
-      items.push_back({rows * ppc, d, t});
+      items.push_back({rows * ppc, d, t, cells_lanes(h) > 0});
     }
     smem = std::max(smem, push_smem_bytes(h->TY, true));
+    csmem = std::max(csmem, cells_smem_bytes(h->TY, true));
+    track |= h->cfg.track_pid != 0;
     maxcells = std::max<int64_t>(maxcells, (int64_t)h->ncells + 1);
     maxbins = std::max<int64_t>(maxbins, (int64_t)h->ntiles * h->nb);
     maxtiles = std::max<int64_t>(maxtiles, (int64_t)h->ntiles + 1);
@@ -1647,12 +1664,16 @@ int batch_layout(pbpic_batch* b) {
     maxacc = std::max<int64_t>(maxacc, 2 * plane_elems(h));  // 16-byte stores of 4 planes
     maxnfe = std::max(maxnfe, h->nfe);
   }
-  std::stable_sort(items.begin(), items.end(), [](const Item& x, const Item& y) { return x.cost > y.cost; });
+  std::stable_sort(items.begin(), items.end(), [](const Item& x, const Item& y) { return x.cells != y.cells ? x.cells : x.cost > y.cost; });
   if (items.size() > (size_t)0x7fffffff) return fail(PBPIC_EINVAL, "too many tiles in the batch");
   b->h_tiles.resize(items.size());
   for (size_t k = 0; k < items.size(); ++k) b->h_tiles[k] = make_int2(items[k].d, items[k].t);
   b->ntiles = (int)items.size();
+  b->ncells_tiles = 0;
+  for (const Item& i : items) b->ncells_tiles += i.cells;
+  b->track = track;
   b->push_smem = smem;
+  b->cells_smem = csmem;
   if (b->d_tiles) cudaFree(b->d_tiles);
   b->d_tiles = nullptr;
   CK(cudaMalloc(&b->d_tiles, std::max<size_t>(1, items.size()) * sizeof(int2)));
@@ -1663,12 +1684,15 @@ int batch_layout(pbpic_batch* b) {
   int per_sm = 1;
   b->compat = false;
   for (pbpic_handle* h : b->dom) b->compat |= h->cfg.compat != 0;
+  const void* cf = b->track ? (const void*)k_push_cells_batched<true> : (const void*)k_push_cells_batched<false>;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cf, PC_THREADS, csmem));
+  b->cells_blocks = std::max(1, std::min(b->ncells_tiles, sms * std::max(1, per_sm)));
   const void* fn = b->groups == 1 ? (b->compat ? (const void*)k_push_batched<float, true, true, 1, true, true>
                                                : (const void*)k_push_batched<float, true, true, 1, false, true>)
                                   : (b->compat ? (const void*)k_push_batched<float, true, true, 2, true, true>
                                                : (const void*)k_push_batched<float, true, true, 2, false, true>);
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, PushThreads<float>::value, smem));
-  b->push_blocks = std::max(1, std::min(b->ntiles, sms * std::max(1, per_sm)));
+  b->push_blocks = std::max(1, std::min(b->ntiles - b->ncells_tiles, sms * std::max(1, per_sm)));
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused_perm_batched<float>, 256, 0));
   b->scatter_blocks = std::max(1, std::min(b->ntiles, sms * std::max(1, per_sm)));
   b->gx_zero = grid_for(maxacc, 256, 1024);
@@ -1702,11 +1726,7 @@ int batch_descriptors(pbpic_batch* b) {
       const int i = h->cur, o = 1 - i;
       pp.src = h->perm;
       pp.cell_o = h->cell[o];
-      pp.dx_o = P<float>(h, o, 0);
-      pp.dy_o = P<float>(h, o, 1);
-      pp.ux_o = P<float>(h, o, 2);
-      pp.uy_o = P<float>(h, o, 3);
-      pp.uz_o = P<float>(h, o, 4);
+      pp.c_o = C<float>(h, o);
       pp.pid_i = h->pid[i];
       pp.pid_o = h->pid[o];
       ScatterParams<float>& sp = b->h_scat[par * D + d];
@@ -1778,16 +1798,20 @@ int batch_enqueue_step(pbpic_batch* b, int par) {
   k_batch_begin<<<dim3(b->gx_zero, D), 256, 0, s>>>(b->d_dom, ctr, ctr + 2);
   CKLAUNCH("k_batch_begin");
   const PushParams<float>* pp = b->d_push + (size_t)par * D;
-  const unsigned nt = PushThreads<float>::value;
-  if (b->groups == 1 && b->compat)
-    k_push_batched<float, true, true, 1, true, true><<<b->push_blocks, nt, b->push_smem, s>>>(pp, b->d_tiles, b->ntiles, ctr);
-  else if (b->groups == 1)
-    k_push_batched<float, true, true, 1, false, true><<<b->push_blocks, nt, b->push_smem, s>>>(pp, b->d_tiles, b->ntiles, ctr);
-  else if (b->compat)
-    k_push_batched<float, true, true, 2, true, true><<<b->push_blocks, nt, b->push_smem, s>>>(pp, b->d_tiles, b->ntiles, ctr);
-  else
-    k_push_batched<float, true, true, 2, false, true><<<b->push_blocks, nt, b->push_smem, s>>>(pp, b->d_tiles, b->ntiles, ctr);
-  CKLAUNCH("k_push_batched");
+  if (b->ncells_tiles > 0) {
+    if (b->track) k_push_cells_batched<true><<<b->cells_blocks, PC_THREADS, b->cells_smem, s>>>(pp, b->d_tiles, b->ncells_tiles, ctr + 3);
+    else k_push_cells_batched<false><<<b->cells_blocks, PC_THREADS, b->cells_smem, s>>>(pp, b->d_tiles, b->ncells_tiles, ctr + 3);
+    CKLAUNCH("k_push_cells_batched");
+  }
+  const int nold = b->ntiles - b->ncells_tiles;
+  if (nold > 0) {
+    auto run = [&](auto kernel) {
+      kernel<<<b->push_blocks, PushThreads<float>::value, b->push_smem, s>>>(pp, b->d_tiles + b->ncells_tiles, nold, ctr);
+    };
+    if (b->groups == 1) b->compat ? run(k_push_batched<float, true, true, 1, true, true>) : run(k_push_batched<float, true, true, 1, false, true>);
+    else b->compat ? run(k_push_batched<float, true, true, 2, true, true>) : run(k_push_batched<float, true, true, 2, false, true>);
+    CKLAUNCH("k_push_batched");
+  }
   k_fused_counts_batched<<<dim3(b->gx_cells, D), 256, 0, s>>>(b->d_fsort);
   CKLAUNCH("k_fused_counts_batched");
   k_scan_batched<<<D, SCB, 0, s>>>(b->d_dom);
@@ -2441,8 +2465,7 @@ int band_extract_sorted(pbpic_handle* h, int y_lo, int y_hi, int my_global, int 
   const int b = h->cur;
   if (total > 0) {
     k_band_out_sorted<T, T><<<std::min(mx, 148 * 16), 256, 0, s>>>(
-        colstart, h->off, mx, h->cfg.my, y_lo, h->cell[b], P<T>(h, b, 0), P<T>(h, b, 1), P<T>(h, b, 2),
-        P<T>(h, b, 3), P<T>(h, b, 4), h->pid[b], my_global, row_offset, (RefRec<T>*)dst,
+        colstart, h->off, mx, h->cfg.my, y_lo, h->cell[b], C<T>(h, b), h->pid[b], my_global, row_offset, (RefRec<T>*)dst,
         h->lazy ? h->perm : nullptr, ((uintptr_t)dst & 15) == 0);
     CKLAUNCH("k_band_out_sorted");
   }
@@ -2462,8 +2485,7 @@ int do_band_extract(pbpic_handle* h, int y_lo, int y_hi, int my_global, int row_
   if (c > 0 && !dst) return fail(PBPIC_EINVAL, "null band destination");
   const int b = h->cur;
   if (h->n > 0 && c > 0) {
-    k_band_out<T, T><<<grid_for(h->n, 256), 256, 0, h->stream>>>(h->n, h->cell[b], P<T>(h, b, 0), P<T>(h, b, 1),
-                                                                 P<T>(h, b, 2), P<T>(h, b, 3), P<T>(h, b, 4),
+    k_band_out<T, T><<<grid_for(h->n, 256), 256, 0, h->stream>>>(h->n, h->cell[b], C<T>(h, b),
                                                                  h->pid[b], h->band_flags, my_global, row_offset,
                                                                  (RefRec<T>*)dst);
     CKLAUNCH("k_band_out");
@@ -2480,8 +2502,8 @@ int do_band_keep(pbpic_handle* h, int y_lo, int y_hi) {
   const int b = h->cur, o = 1 - b;
   if (h->n > 0) {
     k_band_keep<T><<<grid_for(h->n, 256), 256, 0, h->stream>>>(
-        h->n, h->band_flags, h->cell[b], P<T>(h, b, 0), P<T>(h, b, 1), P<T>(h, b, 2), P<T>(h, b, 3), P<T>(h, b, 4),
-        h->pid[b], h->cell[o], P<T>(h, o, 0), P<T>(h, o, 1), P<T>(h, o, 2), P<T>(h, o, 3), P<T>(h, o, 4), h->pid[o]);
+        h->n, h->band_flags, h->cell[b], C<T>(h, b),
+        h->pid[b], h->cell[o], C<T>(h, o), h->pid[o]);
     CKLAUNCH("k_band_keep");
     h->cur = o;
   }
@@ -2500,8 +2522,7 @@ int do_band_append(pbpic_handle* h, const void* src, int64_t n, int my_global, i
   const int b = h->cur;
   CK(cudaMemsetAsync(h->dscalar, 0, 4, s));
   k_band_in<T, T><<<grid_for(n, 256), 256, 0, s>>>((const RefRec<T>*)src, n, my_global, row_offset, h->cfg.mx,
-                                                   h->cfg.my, h->n, h->cell[b], P<T>(h, b, 0), P<T>(h, b, 1),
-                                                   P<T>(h, b, 2), P<T>(h, b, 3), P<T>(h, b, 4), h->pid[b],
+                                                   h->cfg.my, h->n, h->cell[b], C<T>(h, b), h->pid[b],
                                                    (int*)h->dscalar);
   CKLAUNCH("k_band_in");
   int st = 0;
@@ -2578,8 +2599,7 @@ int do_band_replace(pbpic_handle* h, int y_lo, int y_hi, const void* bot, int64_
     // the assembled order is a permutation the next push reads through
     if (nb + nt > 0) {
       k_band_to_soa<T, T><<<grid_for(nb + nt, 256), 256, 0, s>>>(
-          nb, nt, rs, (const RefRec<T>*)bot, (const RefRec<T>*)top, base, h->cell[b], P<T>(h, b, 0), P<T>(h, b, 1),
-          P<T>(h, b, 2), P<T>(h, b, 3), P<T>(h, b, 4), h->pid[b], h->status);
+          nb, nt, rs, (const RefRec<T>*)bot, (const RefRec<T>*)top, base, h->cell[b], C<T>(h, b), h->pid[b], h->status);
       CKLAUNCH("k_band_to_soa");
     }
     const int64_t pcap = std::max<int64_t>(h->cap, 1) + 16;
@@ -2610,9 +2630,7 @@ int do_band_replace(pbpic_handle* h, int y_lo, int y_hi, const void* bot, int64_
   }
   if (total > 0) {
     k_band_assemble<T, T><<<grid_for(total, 256), 256, 0, s>>>(
-        total, rs, (const RefRec<T>*)bot, (const RefRec<T>*)top, h->cell[b], P<T>(h, b, 0), P<T>(h, b, 1),
-        P<T>(h, b, 2), P<T>(h, b, 3), P<T>(h, b, 4), h->pid[b], h->cell[o], P<T>(h, o, 0), P<T>(h, o, 1),
-        P<T>(h, o, 2), P<T>(h, o, 3), P<T>(h, o, 4), h->pid[o], h->status, h->lazy ? h->perm : nullptr);
+        total, rs, (const RefRec<T>*)bot, (const RefRec<T>*)top, h->cell[b], C<T>(h, b), h->pid[b], h->cell[o], C<T>(h, o), h->pid[o], h->status, h->lazy ? h->perm : nullptr);
     CKLAUNCH("k_band_assemble");
   }
   h->cur = o;
@@ -2669,7 +2687,7 @@ int do_energies_rows(pbpic_handle* h, int y_lo, int y_hi, int wall_lo, int wall_
   if (y_lo < 0 || y_hi > h->S || y_lo > y_hi) return fail(PBPIC_EINVAL, "rows outside 0..my");
   cudaStream_t s = h->stream;
   const int b = h->cur;
-  k_kinetic_rows<T, MIXED><<<h->nke, 256, 0, s>>>(h->n, h->cell[b], P<T>(h, b, 2), P<T>(h, b, 3), P<T>(h, b, 4),
+  k_kinetic_rows<T, MIXED><<<h->nke, 256, 0, s>>>(h->n, h->cell[b], C<T>(h, b),
                                                    (T)c.mime, y_lo, std::min(y_hi, c.my), h->ke_part);
   CKLAUNCH("k_kinetic_rows");
   k_field_energy_rows<T><<<h->nfe, 256, 0, s>>>(c.mx, c.my, (const T*)h->ng, y_lo, y_hi, wall_lo, wall_hi,

@@ -140,11 +140,6 @@ PushParams<T> push_params(const pbpic_diff* d, const Slot& s) {
   p.ybc = PBPIC_BC_CONDUCTING;
   p.compat = 0;
   p.cell = v.cell;
-  p.dx = v.c[0];
-  p.dy = v.c[1];
-  p.ux = v.c[2];
-  p.uy = v.c[3];
-  p.uz = v.c[4];
   p.ng = (const T*)d->ng;
   p.cg = nullptr;  // the adjoint kernels gather from the node grid
   p.jacc = d->jacc;
@@ -235,6 +230,7 @@ int step(pbpic_diff* d, const Slot& s, double omega, void* jkeep = nullptr) {
   DiffParams<T> dp;
   memset(&dp, 0, sizeof(dp));
   dp.push = push_params<T>(d, s);
+  for (int k = 0; k < 5; ++k) dp.s[k] = view<T>(d, s).c[k];
   dp.n = d->n;
   dp.nsheet = d->nsheet;
   dp.omega_bg = omega;
@@ -292,8 +288,8 @@ int load(pbpic_diff* d, const pbpic_diff_params* prm) {
   L.lambda = c.lambda;
   L.seed = c.seed;
   View<T> v = view<T>(d, d->work);
-  k_load<T><<<(unsigned)((d->npairs + 255) / 256), 256>>>(L, d->npairs, 0, v.cell, v.c[0], v.c[1], v.c[2], v.c[3],
-                                                           v.c[4], nullptr);
+  k_load<T><<<(unsigned)((d->npairs + 255) / 256), 256>>>(L, d->npairs, 0, v.cell,
+                                                           Soa5<T>{{v.c[0], v.c[1], v.c[2], v.c[3], v.c[4]}}, nullptr);
   DLAUNCH("k_load");
   pic::FieldInit fi;
   fi.kind = pic::LOAD_HARRIS;
@@ -406,6 +402,7 @@ int backward(pbpic_diff* d, double grad[3]) {
       DiffParams<T> dp;
       memset(&dp, 0, sizeof(dp));
       dp.push = push_params<T>(d, d->seg[m]);
+      for (int k = 0; k < 5; ++k) dp.s[k] = view<T>(d, d->seg[m]).c[k];
       dp.n = d->n;
       dp.nsheet = d->nsheet;
       dp.omega_bg = omega;
