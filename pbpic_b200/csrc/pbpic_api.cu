@@ -2449,8 +2449,23 @@ int col_buffers(pbpic_handle* h) {
 template <class T, bool MIXED>
 int band_extract_sorted(pbpic_handle* h, int y_lo, int y_hi, int my_global, int row_offset, void* dst, int64_t cap,
                         int64_t* nout) {
-  TRY(col_buffers(h));
   cudaStream_t s = h->stream;
+  // every row, into a buffer of whole words: no counting on the device, one launch
+  if (y_lo == 0 && y_hi == h->cfg.my && ((uintptr_t)dst & 7) == 0) {
+    if (nout) *nout = h->n;
+    if (h->n > cap) return fail(PBPIC_ECAPACITY, "the band holds more particles than the destination");
+    if (h->n > 0 && !dst) return fail(PBPIC_EINVAL, "null band destination");
+    if (h->n > 0) {
+      const int b = h->cur;
+      k_band_out_all<T><<<grid_for(h->n, 256, 148 * 32), 256, 0, s>>>(h->n, h->cell[b], C<T>(h, b), h->pid[b], my_global,
+                                                                      row_offset, (RefRec<T>*)dst,
+                                                                      h->lazy ? h->perm : nullptr);
+      CKLAUNCH("k_band_out_all");
+    }
+    CK(cudaStreamSynchronize(s));
+    return PBPIC_OK;
+  }
+  TRY(col_buffers(h));
   const int mx = h->cfg.mx;
   int32_t* colstart = h->colbuf;
   k_col_counts<<<grid_for(mx + 1, 256), 256, 0, s>>>(h->off, mx, h->cfg.my, y_lo, y_hi, colstart);
