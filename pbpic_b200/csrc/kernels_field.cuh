@@ -29,7 +29,15 @@ struct FieldParams {
   T* ng;                 // node grid (mx+1) x (my+1) x 8
   T* cg;                 // mixed form: per-cell gather records mx x my x 24 of the push
   double* fe_part;       // per-block field energy partial sums [grid][2]
-  int nblk;              // batched launches: blocks that compute the partials
+  // whole field solve in one launch (k_field_step): the new planes, the next
+  // push's current to clear, and (single domain) the energy row to write
+  T *nex, *ney, *nez, *nbx, *nby, *nbz;
+  void* jnext;
+  const double* ke_part; // kinetic partials of the push, or null
+  int nke;
+  double fe_scale, fb_scale;
+  double* row;           // null: no row (batched domains)
+  int* ticket;           // blocks finished so far (0 between launches)
 };
 
 __device__ __forceinline__ int wrapx(int i, int mx) { return i < 0 ? i + mx : (i >= mx ? i - mx : i); }
@@ -220,6 +228,12 @@ __global__ void k_nodes(FieldParams<T> a) {
 // bilinear coefficients (A, B, C, D) of each of ex ey ez bx by bz over the cell
 // (with PBPIC_CELL_COEF = 0 the 4 nodes themselves), as 6 contiguous 16-byte
 // stores, so the push reads a cell's gather data with 6 loads from one address.
+__device__ __forceinline__ float4 cell_coef(float n00, float n01, float n10, float n11) {
+  const float sx0 = __fadd_rn(n00, n01), sx1 = __fadd_rn(n10, n11);
+  const float sy0 = __fadd_rn(n00, n10), sy1 = __fadd_rn(n01, n11);
+  return make_float4(__fmul_rn(0.25f, __fadd_rn(sx0, sx1)), __fmul_rn(0.5f, __fsub_rn(sx1, sx0)),
+                     __fmul_rn(0.5f, __fsub_rn(sy1, sy0)), __fsub_rn(__fsub_rn(n11, n10), __fsub_rn(n01, n00)));
+}
 __device__ __forceinline__ void cell_record(const FieldParams<float>& a, int cx, int cy) {
   const long long c = (long long)cx * a.my + cy;
   const float4* g00 = reinterpret_cast<const float4*>(a.ng + ((long long)cx * (a.my + 1) + cy) * 8);
@@ -229,18 +243,12 @@ __device__ __forceinline__ void cell_record(const FieldParams<float>& a, int cx,
   float4* r = reinterpret_cast<float4*>(a.cg + c * 24);
 #if PBPIC_CELL_COEF
   // per field: A = mean of the 4 nodes, B = x slope, C = y slope, D = twist
-  auto coef = [](float n00, float n01, float n10, float n11) {
-    const float sx0 = __fadd_rn(n00, n01), sx1 = __fadd_rn(n10, n11);
-    const float sy0 = __fadd_rn(n00, n10), sy1 = __fadd_rn(n01, n11);
-    return make_float4(__fmul_rn(0.25f, __fadd_rn(sx0, sx1)), __fmul_rn(0.5f, __fsub_rn(sx1, sx0)),
-                       __fmul_rn(0.5f, __fsub_rn(sy1, sy0)), __fsub_rn(__fsub_rn(n11, n10), __fsub_rn(n01, n00)));
-  };
-  r[0] = coef(p0.x, p1.x, p2.x, p3.x);
-  r[1] = coef(p0.y, p1.y, p2.y, p3.y);
-  r[2] = coef(p0.z, p1.z, p2.z, p3.z);
-  r[3] = coef(q0.x, q1.x, q2.x, q3.x);
-  r[4] = coef(q0.y, q1.y, q2.y, q3.y);
-  r[5] = coef(q0.z, q1.z, q2.z, q3.z);
+  r[0] = cell_coef(p0.x, p1.x, p2.x, p3.x);
+  r[1] = cell_coef(p0.y, p1.y, p2.y, p3.y);
+  r[2] = cell_coef(p0.z, p1.z, p2.z, p3.z);
+  r[3] = cell_coef(q0.x, q1.x, q2.x, q3.x);
+  r[4] = cell_coef(q0.y, q1.y, q2.y, q3.y);
+  r[5] = cell_coef(q0.z, q1.z, q2.z, q3.z);
 #else
   r[0] = make_float4(p0.x, p0.y, p0.z, q0.x);
   r[1] = make_float4(q0.y, q0.z, p1.x, p1.y);
@@ -348,42 +356,11 @@ __global__ void k_filter_apply(FieldParams<T> a, FilterParams<T> f) {
   }
 }
 
-// Batched domains: grid row blockIdx.y works on domain blockIdx.y.
-template <class T>
-__global__ void k_bhalf_batched(const FieldParams<T>* d) {
-  __shared__ FieldParams<T> a;
-  if (threadIdx.x == 0) a = d[blockIdx.y];
-  __syncthreads();
-  bhalf_body(a);
-}
-template <class T, class Acc>
-__global__ void k_efull_batched(const FieldParams<T>* d) {
-  __shared__ FieldParams<T> a;
-  if (threadIdx.x == 0) a = d[blockIdx.y];
-  __syncthreads();
-  efull_body<T, Acc>(a);
-}
-template <class T>
-__global__ void k_nodes_batched(const FieldParams<T>* d) {
-  __shared__ FieldParams<T> a;
-  __shared__ double red[32];
-  if (threadIdx.x == 0) a = d[blockIdx.y];
-  __syncthreads();
-  if ((int)blockIdx.x < a.nblk) nodes_body(a, red, blockIdx.x, a.nblk);
-}
-static __global__ void k_cell_records_batched(const FieldParams<float>* d) {
-  __shared__ FieldParams<float> a;
-  if (threadIdx.x == 0) a = d[blockIdx.y];
-  __syncthreads();
-  cell_records_body(a, blockIdx.x, gridDim.x);
-}
-
 // Sum the per-tile kinetic and per-block field partials in a fixed order and
 // write one row (electron KE, ion KE, E energy, B energy) of the history.
 // Either pointer may be null, in which case that half of the row is kept.
-static __global__ void k_energy_row(const double* ke_part, int nke, const double* fe_part, int nfe,
-                             double fe_scale, double fb_scale, double* row) {
-  __shared__ double red[32];
+__device__ __forceinline__ void energy_row(const double* ke_part, int nke, const double* fe_part, int nfe,
+                                           double fe_scale, double fb_scale, double* row, double* red) {
   double s[4] = {0, 0, 0, 0};
   if (ke_part)
     for (int i = threadIdx.x; i < nke; i += blockDim.x) {
@@ -392,8 +369,8 @@ static __global__ void k_energy_row(const double* ke_part, int nke, const double
     }
   if (fe_part)
     for (int i = threadIdx.x; i < nfe; i += blockDim.x) {
-      s[2] += fe_part[2 * i];
-      s[3] += fe_part[2 * i + 1];
+      s[2] += __ldcg(fe_part + 2 * i);
+      s[3] += __ldcg(fe_part + 2 * i + 1);
     }
   for (int c = 0; c < 4; ++c) {
     const double t = block_sum(s[c], red);
@@ -403,6 +380,11 @@ static __global__ void k_energy_row(const double* ke_part, int nke, const double
       if (c == 3 && fe_part) row[3] = t * fb_scale;
     }
   }
+}
+static __global__ void k_energy_row(const double* ke_part, int nke, const double* fe_part, int nfe,
+                             double fe_scale, double fb_scale, double* row) {
+  __shared__ double red[32];
+  energy_row(ke_part, nke, fe_part, nfe, fe_scale, fb_scale, row, red);
 }
 
 // One energy row per domain (block blockIdx.x works on domain blockIdx.x),
@@ -419,20 +401,273 @@ struct EnergyRow {
 static __global__ void k_energy_rows_batched(const EnergyRow* d, const int* step) {
   __shared__ double red[32];
   const EnergyRow r = d[blockIdx.x];
-  double* row = r.rows + 4 * (long long)(*step);
-  double s[4] = {0, 0, 0, 0};
-  for (int i = threadIdx.x; i < r.nke; i += blockDim.x) {
-    s[0] += r.ke_part[2 * i];
-    s[1] += r.ke_part[2 * i + 1];
+  energy_row(r.ke_part, r.nke, r.fe_part, r.nfe, r.fe_scale, r.fb_scale, r.rows + 4 * (long long)(*step), red);
+}
+
+// ---------------------------------------------------------------------------
+// The field solve in one launch: B half step, E, B half step, node averages,
+// gather records (mixed form), energy partials, the next push's current
+// cleared and, by the last block to finish, the energy row. A block loads
+// its tile of FX x FY nodes with 4 more rows and columns on each side (each of the four
+// phases needs one neighbour more than the next), updates the planes in
+// shared memory and writes the tile's part to the other set of planes. The values
+// are those of k_bhalf, k_efull, k_bhalf, k_nodes and k_cell_records.
+//
+// Latency-bound: those were six launches of 3-5 us each on the step's second stream, and the
+// current's clearing and the kinetic energy row two more before and after the
+// push. A step on 64x64 cells went from 72 to 38 us with this (14 us) and the counting sort's
+// shorter chain (kernels_sort.cuh: cell_entries), at 128x128 cells and 1 M particles
+// from 94 to 60 us; at 512x256 the solve runs beside the sort either way. Blocks of 512
+// threads, two elements each (256: 18 us). Tile: 46 KB of shared memory in FP64, 960
+// elements loaded for 512 nodes.
+// ---------------------------------------------------------------------------
+constexpr int FT = 512;  // threads of a block
+constexpr int FX = 16, FY = 32, FH = 4, FLX = FX + 2 * FH, FLY = FY + 2 * FH, FN = FLX * FLY;
+constexpr int FNX = FX + 1, FNY = FY + 1;  // nodes of the tile's cells
+
+inline int field_tiles(int mx, int my) { return ((mx + FX - 1) / FX) * ((my + 1 + FY - 1) / FY); }
+
+template <class T>
+struct FieldTile {
+  T f[6][FN];                                // ex ey ez bx by bz
+  T nd[sizeof(T) == 4 ? 6 * FNX * FNY : 1];  // node values (mixed: for the records)
+  double red[32];
+  int last;
+};
+
+__device__ __forceinline__ int wrap_mod(int i, int n) {  // (a few periods off at most)
+  while (i < 0) i += n;
+  while (i >= n) i -= n;
+  return i;
+}
+
+template <class T, class Acc>
+__device__ __forceinline__ void field_step_tile(const FieldParams<T>& a, int bid, FieldTile<T>& s) {
+  const int nty = (a.my + 1 + FY - 1) / FY;
+  const int i0 = (bid / nty) * FX, j0 = (bid % nty) * FY;
+  const bool walls = a.ybc != 0;
+  T(&ex)[FN] = s.f[0];
+  T(&ey)[FN] = s.f[1];
+  T(&ez)[FN] = s.f[2];
+  T(&bx)[FN] = s.f[3];
+  T(&by)[FN] = s.f[4];
+  T(&bz)[FN] = s.f[5];
+  // this thread's elements of the tile: their planes to shared memory, their current for the E step kept
+  constexpr int NK = (FN + FT - 1) / FT;
+  const long long plane = (long long)a.mx * a.S;
+  T jx[NK], jy[NK], jz[NK];
+#pragma unroll
+  for (int k = 0; k < NK; ++k) {
+    const int e = threadIdx.x + k * FT;
+    jx[k] = jy[k] = jz[k] = T(0);
+    if (e >= FN) continue;
+    const int lx = e / FLY, ly = e - lx * FLY;
+    const int gi = wrap_mod(i0 - FH + lx, a.mx);
+    int gj = j0 - FH + ly;
+    if (!walls) gj = wrap_mod(gj, a.my);
+    const bool in = gj >= 0 && gj <= a.my;  // (rows beyond the walls are images, formed where they are read)
+    const long long o = (long long)gi * a.S + gj;
+    ex[e] = in ? a.ex[o] : T(0);
+    ey[e] = in ? a.ey[o] : T(0);
+    ez[e] = in ? a.ez[o] : T(0);
+    bx[e] = in ? a.bx[o] : T(0);
+    by[e] = in ? a.by[o] : T(0);
+    bz[e] = in ? a.bz[o] : T(0);
+    if (in && lx >= 2 && ly >= 2 && lx < FLX - 2 && ly < FLY - 2) {
+      jx[k] = (T)(jval<Acc>(a.jacc, o) * a.jscale[0]);
+      jy[k] = (T)(jval<Acc>(a.jacc, plane + o) * a.jscale[1]);
+      jz[k] = (T)(jval<Acc>(a.jacc, 2 * plane + o) * a.jscale[2]);
+    }
   }
-  for (int i = threadIdx.x; i < r.nfe; i += blockDim.x) {
-    s[2] += r.fe_part[2 * i];
-    s[3] += r.fe_part[2 * i + 1];
+  __syncthreads();
+  // half-row component at local e, row j or j - 1 (half_row, with the image of walls)
+  auto half_at = [&](const T* f, int e, int j, T odd) -> T {
+    if (walls && j >= a.my) return odd * f[e - (j - (a.my - 1))];
+    if (walls && j < 0) return odd * f[e - j];
+    return f[e];
+  };
+  auto bhalf = [&](int lo) {
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+      const int e = threadIdx.x + k * FT, lx = e / FLY, ly = e - lx * FLY, j = j0 - FH + ly;
+      if (lx < lo || ly < lo || lx >= FLX - lo || ly >= FLY - lo) continue;
+      if (walls && (j < 0 || j > a.my)) continue;
+      const T ezj = half_at(ez, e, j, T(-1)), ezm = half_at(ez, e - 1, j - 1, T(-1));
+      const T d = (ezj - ezm) * a.idy;
+      bx[e] = bx[e] - a.dth * d;
+      if (!walls || j < a.my) {
+        const T dezdx = (ez[e] - ez[e - FLY]) * a.idx;
+        by[e] = by[e] + a.dth * dezdx;
+        const T dexdy = (ex[e + 1] - ex[e]) * a.idy;
+        const T deydx = (ey[e + FLY] - ey[e]) * a.idx;
+        bz[e] = bz[e] + a.dth * (dexdy - deydx);
+      }
+    }
+    __syncthreads();
+  };
+  bhalf(1);
+#pragma unroll
+  for (int k = 0; k < NK; ++k) {
+    const int e = threadIdx.x + k * FT, lx = e / FLY, ly = e - lx * FLY, j = j0 - FH + ly;
+    if (lx < 2 || ly < 2 || lx >= FLX - 2 || ly >= FLY - 2) continue;
+    if (walls && (j < 0 || j > a.my)) continue;
+    if (walls && (j == 0 || j == a.my)) {
+      ex[e] = T(0);  // tangential E on a perfect conductor
+    } else {
+      const T bzj = half_at(bz, e, j, T(1)), bzm = half_at(bz, e - 1, j - 1, T(1));
+      const T dbzdy = (bzj - bzm) * a.idy;
+      ex[e] = ex[e] + a.cdt * (dbzdy - jx[k]);
+    }
+    if (!walls || j < a.my) {
+      const T dbzdx = (bz[e] - bz[e - FLY]) * a.idx;
+      ey[e] = ey[e] - a.cdt * (dbzdx + jy[k]);
+      const T dbydx = (by[e + FLY] - by[e]) * a.idx;
+      const T dbxdy = (bx[e + 1] - bx[e]) * a.idy;
+      ez[e] = ez[e] + a.cdt * (dbydx - dbxdy - jz[k]);
+    }
   }
-  for (int c = 0; c < 4; ++c) {
-    const double t = block_sum(s[c], red);
-    if (threadIdx.x == 0) row[c] = c == 2 ? t * r.fe_scale : (c == 3 ? t * r.fb_scale : t);
+  __syncthreads();
+  bhalf(3);
+  // the tile's planes; rows that no boundary uses (periodic row my, the half rows' row my) are kept
+  for (int e = threadIdx.x; e < FX * FY; e += FT) {
+    const int gi = i0 + e / FY, gj = j0 + e % FY;
+    if (gi >= a.mx || gj > a.my) continue;
+    const int l = (FH + e / FY) * FLY + FH + e % FY;
+    const long long o = (long long)gi * a.S + gj;
+    const bool node_ok = walls || gj < a.my, half_ok = gj < a.my;
+    a.nex[o] = node_ok ? ex[l] : a.ex[o];
+    a.nbx[o] = node_ok ? bx[l] : a.bx[o];
+    a.ney[o] = half_ok ? ey[l] : a.ey[o];
+    a.nez[o] = half_ok ? ez[l] : a.ez[o];
+    a.nby[o] = half_ok ? by[l] : a.by[o];
+    a.nbz[o] = half_ok ? bz[l] : a.bz[o];
+    if (a.jnext) {
+      long long* z = reinterpret_cast<long long*>(a.jnext);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) z[c * plane + o] = 0;
+    }
   }
+  // node averages (node_at) and energies
+  double se = 0.0, sb = 0.0;
+  for (int e = threadIdx.x; e < FNX * FNY; e += FT) {
+    const int nx = e / FNY, ny = e - nx * FNY, gi = i0 + nx, b = j0 + ny;
+    if (gi > a.mx || b > a.my) continue;
+    const int l = (FH + nx) * FLY + FH + ny, m = l - FLY;
+    T v[6];
+    v[0] = (ex[l] + ex[m]) * T(0.5);
+    v[3] = (bx[l] + bx[m]) * T(0.5);
+    v[1] = (half_at(ey, l, b, T(1)) + half_at(ey, l - 1, b - 1, T(1))) * T(0.5);
+    v[4] = (half_at(by, l, b, T(-1)) + half_at(by, l - 1, b - 1, T(-1))) * T(0.5);
+    v[2] = (half_at(ez, l, b, T(-1)) + half_at(ez, m, b, T(-1)) + half_at(ez, l - 1, b - 1, T(-1)) +
+            half_at(ez, m - 1, b - 1, T(-1))) * T(0.25);
+    v[5] = (half_at(bz, l, b, T(1)) + half_at(bz, m, b, T(1)) + half_at(bz, l - 1, b - 1, T(1)) +
+            half_at(bz, m - 1, b - 1, T(1))) * T(0.25);
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) s.nd[k * FNX * FNY + e] = v[k];
+    }
+    if (ny < FY && (nx < FX || gi == a.mx)) {
+      T* g = a.ng + ((long long)gi * (a.my + 1) + b) * 8;
+      g[0] = v[0];
+      g[1] = v[1];
+      g[2] = v[2];
+      g[3] = T(0);
+      g[4] = v[3];
+      g[5] = v[4];
+      g[6] = v[5];
+      g[7] = T(0);
+      if (gi < a.mx && (walls || b < a.my)) {
+        const double w = (walls && (b == 0 || b == a.my)) ? 0.5 : 1.0;
+        const T e2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2], b2 = v[3] * v[3] + v[4] * v[4] + v[5] * v[5];
+        se += w * (double)e2;
+        sb += w * (double)b2;
+      }
+    }
+  }
+  const double te = block_sum(se, s.red), tb = block_sum(sb, s.red);  // (barriers: the nodes are in place)
+  if (threadIdx.x == 0) {
+    a.fe_part[2 * bid] = te;
+    a.fe_part[2 * bid + 1] = tb;
+  }
+  if constexpr (sizeof(T) == 4) {
+    for (int e = threadIdx.x; e < FX * FY; e += FT) {
+      const int cx = i0 + e / FY, cy = j0 + e % FY;
+      if (cx >= a.mx || cy >= a.my) continue;
+      const int n = (e / FY) * FNY + e % FY;
+      float4* r = reinterpret_cast<float4*>(a.cg + ((long long)cx * a.my + cy) * 24);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const T* v = s.nd + k * FNX * FNY + n;
+        r[k] = cell_coef(v[0], v[1], v[FNY], v[FNY + 1]);
+      }
+    }
+  }
+}
+
+template <class T, class Acc>
+__global__ void __launch_bounds__(FT) k_field_step(FieldParams<T> a) {
+  __shared__ FieldTile<T> s;
+  field_step_tile<T, Acc>(a, blockIdx.x, s);
+  // the last block to finish adds up every block's partials, in the order of k_energy_row
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s.last = atomicAdd(a.ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!s.last) return;
+  __threadfence();
+  energy_row(a.ke_part, a.nke, a.fe_part, gridDim.x, a.fe_scale, a.fb_scale, a.row, s.red);
+  if (threadIdx.x == 0) *a.ticket = 0;
+}
+
+// Batched domains: grid row blockIdx.y works on domain blockIdx.y.
+template <class T>
+__global__ void k_bhalf_batched(const FieldParams<T>* d) {
+  __shared__ FieldParams<T> a;
+  if (threadIdx.x == 0) a = d[blockIdx.y];
+  __syncthreads();
+  bhalf_body(a);
+}
+template <class T, class Acc>
+__global__ void k_efull_batched(const FieldParams<T>* d) {
+  __shared__ FieldParams<T> a;
+  if (threadIdx.x == 0) a = d[blockIdx.y];
+  __syncthreads();
+  efull_body<T, Acc>(a);
+}
+// (Energy partials by field tile and in its order, as k_field_step forms them: a
+// batched domain's energy history has the bits of the same domain stepped alone.)
+template <class T>
+__global__ void __launch_bounds__(256) k_nodes_batched(const FieldParams<T>* d) {
+  __shared__ FieldParams<T> a;
+  __shared__ double red[32];
+  if (threadIdx.x == 0) a = d[blockIdx.y];
+  __syncthreads();
+  const int nty = (a.my + 1 + FY - 1) / FY;
+  if ((int)blockIdx.x >= ((a.mx + FX - 1) / FX) * nty) return;
+  const int i0 = ((int)blockIdx.x / nty) * FX, j0 = ((int)blockIdx.x % nty) * FY;
+  double se = 0.0, sb = 0.0;
+  for (int e = threadIdx.x; e < FNX * FNY; e += blockDim.x) {
+    const int nx = e / FNY, ny = e - nx * FNY, gi = i0 + nx, b = j0 + ny;
+    if (gi > a.mx || b > a.my || ny >= FY || !(nx < FX || gi == a.mx)) continue;
+    T e2, b2;
+    node_at(a, gi, b, e2, b2);
+    if (gi < a.mx && (a.ybc != 0 || b < a.my)) {
+      const double w = (a.ybc != 0 && (b == 0 || b == a.my)) ? 0.5 : 1.0;
+      se += w * (double)e2;
+      sb += w * (double)b2;
+    }
+  }
+  const double te = block_sum(se, red), tb = block_sum(sb, red);
+  if (threadIdx.x == 0) {
+    a.fe_part[2 * blockIdx.x] = te;
+    a.fe_part[2 * blockIdx.x + 1] = tb;
+  }
+}
+static __global__ void k_cell_records_batched(const FieldParams<float>* d) {
+  __shared__ FieldParams<float> a;
+  if (threadIdx.x == 0) a = d[blockIdx.y];
+  __syncthreads();
+  cell_records_body(a, blockIdx.x, gridDim.x);
 }
 
 }  // namespace pbd

@@ -283,35 +283,6 @@ namespace pbd {
 //                  + [earlier particles of its own tile in the cell],
 // where "earlier" is array order, i.e. tile order then position in the tile.
 
-// Tiles whose window contains cell (cx, cy): the owners of its 3x3 neighbours.
-__device__ __forceinline__ int tiles_of_cell(int cx, int cy, int mx, int my, int ybc, int ty, int tpc, int* tl) {
-  int n = 0;
-#pragma unroll
-  for (int a = -1; a <= 1; ++a) {
-    int x = cx + a;
-    x = x < 0 ? x + mx : (x >= mx ? x - mx : x);
-#pragma unroll
-    for (int b = -1; b <= 1; ++b) {
-      int y = cy + b;
-      if (ybc == 0) {
-        y = y < 0 ? y + my : (y >= my ? y - my : y);
-      } else if (y < 0 || y >= my) {
-        continue;
-      }
-      const int tt = x * tpc + y / ty;
-      bool dup = false;
-      for (int k = 0; k < n; ++k) dup |= tl[k] == tt;
-      if (!dup) tl[n++] = tt;
-    }
-  }
-  return n;
-}
-
-__device__ __forceinline__ int bin_in_tile(int cx, int cy, int tt, int mx, int my, int ybc, int ty, int tpc) {
-  const int ixt = tt / tpc, y0 = (tt - ixt * tpc) * ty, y1 = min(y0 + ty, my);
-  return window_bin(cx, cy, ixt, y0, y1, ty, mx, my, ybc);
-}
-
 struct FusedSortParams {
   int mx, my, ybc, ty, tpc, ntiles, nb;
   const int32_t* tilecnt;  // [ntiles][nb] from the push
@@ -320,105 +291,162 @@ struct FusedSortParams {
   int32_t* base;           // [ntiles][nb] first slot of each (tile, bin)
 };
 
-// A cell whose 3x3 neighbours need no wrap or wall: the tiles whose windows hold it are the
-// tile rows (cy-1)/ty .. (cy+1)/ty of columns cx-1, cx, cx+1, and its bin in the tile of column
-// cx+dx and tile row tr is (1-dx, cy - tr*ty + 1) -- the same tiles and bins tiles_of_cell and
-// bin_in_tile find, in tile order (column, then row).
-__device__ __forceinline__ bool interior_cell(int cx, int cy, int mx, int my) {
-  return cx >= 1 && cx <= mx - 2 && cy >= 1 && cy <= my - 2;
-}
-__device__ __forceinline__ int64_t interior_bin_index(const FusedSortParams& a, int cx, int cy, int dx, int tr) {
-  return ((int64_t)(cx + dx) * a.tpc + tr) * a.nb + (1 - dx) * (a.ty + 2) + (cy - tr * a.ty + 1);
+// The (tile, bin) entries of a cell: the tiles whose windows hold it are those of
+// columns cx - 1, cx, cx + 1 (wrapped) and of the tile rows of rows cy - 1, cy, cy + 1
+// (wrapped, or none beyond a wall). Entry (i, j), i and j in tile order, is at col[i] +
+// row[j] of the [ntiles][nb] tables; a tile row that repeats an earlier one has row < 0. No
+// arrays indexed at run time and two divisions a cell: with the tiles searched for one by one, as
+// edge cells used to be, every warp of a 64-row column waited for its two edge cells
+// (counts 10.6 us and offsets 12.2 us on 64x64 cells).
+struct CellEntries {
+  int64_t col[3];
+  int row[3];
+};
+__device__ __forceinline__ CellEntries cell_entries(const FusedSortParams& a, int cx, int cy) {
+  CellEntries e;
+  // columns in increasing order; bin column 1 for the cell's own, 0 for the column
+  // after the cell's (the cell is before it), 2 for the column before it
+  const int xm = cx == 0 ? a.mx - 1 : cx - 1, xp = cx == a.mx - 1 ? 0 : cx + 1;
+  const int64_t tn = (int64_t)a.tpc * a.nb;
+  const int w = a.ty + 2;
+  const int64_t em = xm * tn + 2 * w, e0 = cx * tn + w, ep = xp * tn;
+  const bool first = cx == 0, last = cx == a.mx - 1;  // order: 0 1 mx-1, or 0 mx-2 mx-1
+  e.col[0] = first ? e0 : (last ? ep : em);
+  e.col[1] = first ? ep : (last ? em : e0);
+  e.col[2] = first ? em : (last ? e0 : ep);
+  const int t0 = cy / a.ty, r0 = cy - t0 * a.ty;
+  const bool top = cy == a.my - 1;
+  // tile row and window row (cy - y0 + 1, wrapped) of the neighbour rows' tiles
+  int tm = r0 > 0 ? t0 : t0 - 1, bm = cy - tm * a.ty + 1;
+  int tp = (r0 < a.ty - 1 && !top) ? t0 : t0 + 1, bp = cy - tp * a.ty + 1;
+  if (cy == 0) {
+    tm = a.ybc == 0 ? a.tpc - 1 : t0;
+    bm = cy - tm * a.ty + 1 + (a.ybc == 0 ? a.my : 0);
+  }
+  if (top) {
+    tp = a.ybc == 0 ? 0 : t0;
+    bp = cy - tp * a.ty + 1 - (a.ybc == 0 ? a.my : 0);
+  }
+  const int vm = tm * a.nb + bm, v0 = t0 * a.nb + r0 + 1, vp = tp * a.nb + bp;
+  // in increasing order of the tile row: wrapped rows come last (row 0's) or first (row my - 1's)
+  const bool mlast = tm > t0, pfirst = tp < t0;
+  const int um = tm == t0 ? -1 : vm, up = (tp == t0 || (tp == tm && um >= 0)) ? -1 : vp;
+  e.row[0] = pfirst ? up : (mlast ? v0 : um);
+  e.row[1] = pfirst ? um : (mlast ? up : v0);
+  e.row[2] = pfirst ? v0 : (mlast ? um : up);
+  return e;
 }
 
-__device__ __forceinline__ void fused_counts_body(const FusedSortParams& a) {
-  const int64_t ncells = (int64_t)a.mx * a.my;
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c <= ncells; c += (int64_t)gridDim.x * blockDim.x) {
-    if (c == ncells) {
-      a.counts[c] = 0;
-      continue;
-    }
-    const int cx = (int)(c / a.my), cy = (int)(c - (int64_t)cx * a.my);
-    int32_t s = 0;
-    if (interior_cell(cx, cy, a.mx, a.my)) {
-      const int tlo = (cy - 1) / a.ty, thi = (cy + 1) / a.ty;
-      for (int dx = -1; dx <= 1; ++dx)
-        for (int tr = tlo; tr <= thi; ++tr) s += a.tilecnt[interior_bin_index(a, cx, cy, dx, tr)];
-    } else {
-      int tl[9];
-      const int n = tiles_of_cell(cx, cy, a.mx, a.my, a.ybc, a.ty, a.tpc, tl);
-      for (int k = 0; k < n; ++k) {
-        const int b = bin_in_tile(cx, cy, tl[k], a.mx, a.my, a.ybc, a.ty, a.tpc);
-        if (b >= 0) s += a.tilecnt[(int64_t)tl[k] * a.nb + b];
-      }
-    }
-    a.counts[c] = s;
+__device__ __forceinline__ int32_t fused_count(const FusedSortParams& a, int c) {
+  const int cx = c / a.my, cy = c - cx * a.my;
+  const CellEntries e = cell_entries(a, cx, cy);
+  int32_t v[9], s = 0;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) v[k] = e.row[k % 3] >= 0 ? __ldg(a.tilecnt + e.col[k / 3] + e.row[k % 3]) : 0;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) s += v[k];
+  return s;
+}
+
+// First slots of the (tile, bin) entries of cell c, whose particles start at `o`: a running sum in tile order.
+__device__ __forceinline__ void fused_slots(const FusedSortParams& a, int c, int32_t o) {
+  const int cx = c / a.my, cy = c - cx * a.my;
+  const CellEntries e = cell_entries(a, cx, cy);
+  int32_t v[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) v[k] = e.row[k % 3] >= 0 ? __ldg(a.tilecnt + e.col[k / 3] + e.row[k % 3]) : 0;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    if (e.row[k % 3] >= 0) a.base[e.col[k / 3] + e.row[k % 3]] = o;
+    o += v[k];
   }
 }
 
-__device__ __forceinline__ void fused_base_body(const FusedSortParams& a) {
-  const int64_t n = (int64_t)a.ntiles * a.nb;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-    const int tt = (int)(e / a.nb), b = (int)(e - (int64_t)tt * a.nb);
-    int32_t base = 0;
-    if (a.tilecnt[e] > 0) {
-      const int ixt = tt / a.tpc, y0 = (tt - ixt * a.tpc) * a.ty;
-      const int bx = b / (a.ty + 2), by = b - bx * (a.ty + 2);
-      int cx = ixt - 1 + bx;
-      cx = cx < 0 ? cx + a.mx : (cx >= a.mx ? cx - a.mx : cx);
-      int cy = y0 - 1 + by;
-      if (a.ybc == 0) cy = cy < 0 ? cy + a.my : (cy >= a.my ? cy - a.my : cy);
-      const int64_t c = (int64_t)cx * a.my + cy;
-      base = a.off[c];
-      int tl[9];
-      const int nt = tiles_of_cell(cx, cy, a.mx, a.my, a.ybc, a.ty, a.tpc, tl);
-      for (int k = 0; k < nt; ++k) {
-        if (tl[k] >= tt) continue;
-        const int b2 = bin_in_tile(cx, cy, tl[k], a.mx, a.my, a.ybc, a.ty, a.tpc);
-        if (b2 >= 0) base += a.tilecnt[(int64_t)tl[k] * a.nb + b2];
-      }
-    }
-    a.base[e] = base;
+// The fused sort's tables in two launches. k_counts_scan: the cell counts of a chunk of
+// CS_TILE cells and their exclusive scan within it, and the chunk's total.
+// k_fused_offsets: every block sums the totals before its chunk itself (they are
+// a few KB in L2), completes the chunk's offsets and gives each (tile, bin) its
+// first slot (the offset plus the cell's particles in earlier tiles) and each tile its position range. `scanned`: the totals are
+// already prefix sums (more than CS_MAXCHUNKS chunks).
+//
+// Latency-bound, 5-6 us each on 64x64 cells; counts, chunk scan, scan of the totals, offsets
+// and tile ranges were five launches of together 41 us there. Chunks of 1024 cells
+// so that 131 thousand cells still fill 128 blocks.
+constexpr int CS_BT = 256, CS_IPT = 4, CS_TILE = CS_BT * CS_IPT;
+constexpr int CS_MAXCHUNKS = 8192;
+
+static __global__ void __launch_bounds__(CS_BT) k_counts_scan(FusedSortParams a, int32_t* sums) {
+  __shared__ int32_t buf[CS_TILE];
+  __shared__ int32_t ws[CS_BT / 32];
+  const int t = threadIdx.x;
+  const int64_t ncells = (int64_t)a.mx * a.my, base = (int64_t)blockIdx.x * CS_TILE;
+#pragma unroll
+  for (int k = 0; k < CS_IPT; ++k) {
+    const int64_t c = base + k * CS_BT + t;
+    const int32_t v = c < ncells ? fused_count(a, (int)c) : 0;
+    buf[k * CS_BT + t] = v;
+    if (c <= ncells) a.counts[c] = v;
   }
+  __syncthreads();
+  int32_t v[CS_IPT], s = 0;
+#pragma unroll
+  for (int k = 0; k < CS_IPT; ++k) {
+    v[k] = s;
+    s += buf[t * CS_IPT + k];
+  }
+  int32_t inc = s;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int32_t y = __shfl_up_sync(FULL, inc, d);
+    if ((int)lane_id() >= d) inc += y;
+  }
+  if (lane_id() == 31) ws[t >> 5] = inc;
+  __syncthreads();
+  int32_t before = 0;
+#pragma unroll
+  for (int k = 0; k < CS_BT / 32; ++k) before += k < (t >> 5) ? ws[k] : 0;
+  const int32_t excl = before + inc - s;
+#pragma unroll
+  for (int k = 0; k < CS_IPT; ++k) buf[t * CS_IPT + k] = excl + v[k];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < CS_IPT; ++k) {
+    const int64_t c = base + k * CS_BT + t;
+    if (c <= ncells) a.off[c] = buf[k * CS_BT + t];
+  }
+  if (t == CS_BT - 1) sums[blockIdx.x] = before + inc;
 }
 
-static __global__ void k_fused_counts(FusedSortParams a) { fused_counts_body(a); }
-
-// After the chunk scan of the counts (k_scan_local) and the scan of the chunk
-// totals, one thread per cell: the cell's offset (its chunk's prefix added)
-// and the first slot of each (tile, bin) that holds the cell (the offset plus
-// the cell's particles in earlier tiles, as fused_base_body).
-static __global__ void k_fused_offsets(FusedSortParams a, const int32_t* sums) {
-  const int64_t ncells = (int64_t)a.mx * a.my;
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c <= ncells; c += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t o = a.off[c] + sums[c / SCAN_TILE];
+static __global__ void __launch_bounds__(CS_BT) k_fused_offsets(FusedSortParams a, const int32_t* sums, bool scanned,
+                                                                int32_t* tile_off) {
+  __shared__ int32_t ws[CS_BT / 32];
+  const int t = threadIdx.x;
+  const int64_t ncells = (int64_t)a.mx * a.my, base = (int64_t)blockIdx.x * CS_TILE;
+  int32_t prefix = 0;
+  if (scanned) {
+    prefix = sums[blockIdx.x];
+  } else {
+    for (int k = t; k < (int)blockIdx.x; k += CS_BT) prefix += sums[k];
+    prefix = __reduce_add_sync(FULL, prefix);
+    if (lane_id() == 0) ws[t >> 5] = prefix;
+    __syncthreads();
+    prefix = 0;
+#pragma unroll
+    for (int k = 0; k < CS_BT / 32; ++k) prefix += ws[k];
+  }
+#pragma unroll
+  for (int k = 0; k < CS_IPT; ++k) {
+    const int64_t c = base + k * CS_BT + t;
+    if (c > ncells) continue;
+    const int32_t o = a.off[c] + prefix;
     a.off[c] = o;
-    if (c == ncells) continue;
-    const int cx = (int)(c / a.my), cy = (int)(c - (int64_t)cx * a.my);
-    if (interior_cell(cx, cy, a.mx, a.my)) {  // the (tile, bin) entries in tile order: a running sum
-      const int tlo = (cy - 1) / a.ty, thi = (cy + 1) / a.ty;
-      int32_t before = o;
-      for (int dx = -1; dx <= 1; ++dx)
-        for (int tr = tlo; tr <= thi; ++tr) {
-          const int64_t e = interior_bin_index(a, cx, cy, dx, tr);
-          a.base[e] = before;
-          before += a.tilecnt[e];
-        }
+    if (c == ncells) {
+      tile_off[a.ntiles] = o;
       continue;
     }
-    int tl[9], bl[9], cl[9];
-    const int nt = tiles_of_cell(cx, cy, a.mx, a.my, a.ybc, a.ty, a.tpc, tl);
-    for (int k = 0; k < nt; ++k) {
-      bl[k] = bin_in_tile(cx, cy, tl[k], a.mx, a.my, a.ybc, a.ty, a.tpc);
-      cl[k] = bl[k] >= 0 ? a.tilecnt[(int64_t)tl[k] * a.nb + bl[k]] : 0;
-    }
-    for (int k = 0; k < nt; ++k) {
-      if (bl[k] < 0) continue;
-      int32_t before = o;
-      for (int j = 0; j < nt; ++j)
-        if (tl[j] < tl[k]) before += cl[j];
-      a.base[(int64_t)tl[k] * a.nb + bl[k]] = before;
-    }
+    const int cx = (int)c / a.my, cy = (int)c - cx * a.my;
+    if (cy % a.ty == 0) tile_off[cx * a.tpc + cy / a.ty] = o;
+    fused_slots(a, (int)c, o);
   }
 }
 
@@ -426,14 +454,17 @@ static __global__ void k_fused_counts_batched(const FusedSortParams* d) {
   __shared__ FusedSortParams a;
   if (threadIdx.x == 0) a = d[blockIdx.y];
   __syncthreads();
-  fused_counts_body(a);
+  const int ncells = a.mx * a.my;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncells; c += gridDim.x * blockDim.x)
+    a.counts[c] = c == ncells ? 0 : fused_count(a, c);
 }
 
 static __global__ void k_fused_base_batched(const FusedSortParams* d) {
   __shared__ FusedSortParams a;
   if (threadIdx.x == 0) a = d[blockIdx.y];
   __syncthreads();
-  fused_base_body(a);
+  const int ncells = a.mx * a.my;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += gridDim.x * blockDim.x) fused_slots(a, c, a.off[c]);
 }
 
 template <class T>

@@ -149,10 +149,15 @@ struct pbpic_handle {
   int32_t* pid[2] = {nullptr, nullptr};
   int cur = 0;
   void* f[6] = {nullptr};
+  void* f2[6] = {nullptr};  // the planes the next one-launch field solve writes (then swapped with f)
   void* ng = nullptr;
   void* cg = nullptr;  // mixed form: per-cell gather records of the push (k_cell_records after k_nodes)
   void* jacc = nullptr;
+  void* jacc2 = nullptr;   // the next push's current; clear when j2_clear (the field solve clears it)
+  bool j2_clear = false;
   int32_t *counts = nullptr, *off = nullptr, *tile_off = nullptr;
+  int32_t* tile_off2 = nullptr;  // written by the fused sort while its ranking reads tile_off (then swapped)
+  int* ticket = nullptr;         // k_field_step's count of finished blocks
   double *ke_part = nullptr, *fe_part = nullptr;
   int nfe = 0, nke = 0;
   double* hist = nullptr;
@@ -165,7 +170,8 @@ struct pbpic_handle {
   bool sorted = false;
   bool fused_ok = false;    // grid admits the fused counting sort (distinct window cells)
   bool hist_valid = false;  // the last push counted new cells per tile on a sorted array
-  bool defer_sort = false;  // pbpic_step: the push leaves its fused sort to run beside the field solve
+  bool defer_sort = false;  // pbpic_step: the push leaves its fused sort to run beside the field solve,
+                            // and its kinetic energies to the field solve's energy row
   cudaStream_t side = nullptr;                       // pbpic_step: the field solve's stream
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;  // pbpic_step: push -> field solve, field solve -> next
   // The fused sort leaves the particle data in place and writes perm (sorted
@@ -386,6 +392,18 @@ FieldParams<T> field_params(pbpic_handle* h) {
   a.ng = (T*)h->ng;
   a.cg = (T*)h->cg;
   a.fe_part = h->fe_part;
+  a.nex = (T*)h->f2[0];
+  a.ney = (T*)h->f2[1];
+  a.nez = (T*)h->f2[2];
+  a.nbx = (T*)h->f2[3];
+  a.nby = (T*)h->f2[4];
+  a.nbz = (T*)h->f2[5];
+  a.jnext = nullptr;
+  a.ke_part = nullptr;
+  a.nke = 0;
+  a.fe_scale = a.fb_scale = 0;
+  a.row = nullptr;
+  a.ticket = h->ticket;
   return a;
 }
 
@@ -394,7 +412,7 @@ double fb_scale(const pbpic_config& c) { return 0.5 * c.mime / (c.cva * c.cva * 
 
 // ------------------------------------------------------------ operations
 template <class T, bool MIXED>
-int nodes_and_field_energy(pbpic_handle* h, int row) {
+int nodes_and_field_energy(pbpic_handle* h, int row, bool ke = false) {
   TRY(ensure_hist(h, row + 1));
   FieldParams<T> a = field_params<T, MIXED>(h);
   k_nodes<T><<<h->nfe, 256, 0, h->stream>>>(a);
@@ -403,7 +421,7 @@ int nodes_and_field_energy(pbpic_handle* h, int row) {
     k_cell_records<<<h->nfe, 256, 0, h->stream>>>(a);
     CKLAUNCH("k_cell_records");
   }
-  k_energy_row<<<1, 256, 0, h->stream>>>(nullptr, 0, h->fe_part, h->nfe, fe_scale(h->cfg), fb_scale(h->cfg),
+  k_energy_row<<<1, 256, 0, h->stream>>>(ke ? h->ke_part : nullptr, h->ntiles, h->fe_part, h->nfe, fe_scale(h->cfg), fb_scale(h->cfg),
                                           h->hist + (size_t)row * 4);
   CKLAUNCH("k_energy_row");
   return PBPIC_OK;
@@ -541,7 +559,9 @@ int do_push(pbpic_handle* h) {
   if (autosort && !h->sorted) TRY((do_sort<T, MIXED>(h)));
   cudaStream_t s = h->stream;
   TRY(ensure_hist(h, h->itime + 2));
-  CK(cudaMemsetAsync(h->jacc, 0, (size_t)4 * plane_elems(h) * 8, s));
+  if (h->j2_clear) std::swap(h->jacc, h->jacc2);
+  else CK(cudaMemsetAsync(h->jacc, 0, (size_t)4 * plane_elems(h) * 8, s));
+  h->j2_clear = false;
   PushParams<T> p = push_params<T, MIXED>(h);
   const size_t smem = push_smem_bytes(h->TY, MIXED);
   if (h->TY > 64) return fail(PBPIC_ESTATE, "k_push: tiles have at most 64 rows");
@@ -575,8 +595,10 @@ int do_push(pbpic_handle* h) {
     else k_push<T, MIXED, false, true><<<h->ntiles, nt, smem, s>>>(p);
     CKLAUNCH("k_push");
   }
-  k_energy_row<<<1, 256, 0, s>>>(h->ke_part, h->ntiles, nullptr, 0, 0, 0, h->hist + (size_t)(h->itime + 1) * 4);
-  CKLAUNCH("k_energy_row");
+  if (!h->defer_sort) {
+    k_energy_row<<<1, 256, 0, s>>>(h->ke_part, h->ntiles, nullptr, 0, 0, 0, h->hist + (size_t)(h->itime + 1) * 4);
+    CKLAUNCH("k_energy_row");
+  }
   h->hist_valid = hist;
   h->sorted = false;
   if (autosort && !h->defer_sort) TRY((do_fused_sort<T, MIXED>(h)));
@@ -600,16 +622,14 @@ int do_fused_sort(pbpic_handle* h) {
   f.counts = h->counts;
   f.off = h->off;
   f.base = h->tbase;
-  // cell counts; their chunk scan into the offsets; the scan of the chunk
-  // totals; one pass per cell adding the chunk prefixes and writing the
-  // (tile, bin) first slots
-  k_fused_counts<<<grid_for((int64_t)h->ncells + 1, 256), 256, 0, s>>>(f);
-  CKLAUNCH("k_fused_counts");
-  const int64_t nchunks = ((int64_t)h->ncells + 1 + SCAN_TILE - 1) / SCAN_TILE;
-  k_scan_local<<<(unsigned)nchunks, SCAN_BT, 0, s>>>(h->counts, h->off, (int64_t)h->ncells + 1, h->scan_scratch);
-  CKLAUNCH("k_scan_local");
-  TRY(scan_excl(s, h->scan_scratch, nchunks, h->scan_scratch + nchunks + 1));
-  k_fused_offsets<<<grid_for((int64_t)h->ncells + 1, 256), 256, 0, s>>>(f, h->scan_scratch);
+  // cell counts and their chunk scan; then the offsets, the (tile, bin) first
+  // slots and the new tile ranges (the ranking still reads the push's)
+  const int64_t nchunks = ((int64_t)h->ncells + 1 + CS_TILE - 1) / CS_TILE;
+  k_counts_scan<<<(unsigned)nchunks, CS_BT, 0, s>>>(f, h->scan_scratch);
+  CKLAUNCH("k_counts_scan");
+  const bool scanned = nchunks > CS_MAXCHUNKS;
+  if (scanned) TRY(scan_excl(s, h->scan_scratch, nchunks, h->scan_scratch + nchunks + 1));
+  k_fused_offsets<<<(unsigned)nchunks, CS_BT, 0, s>>>(f, h->scan_scratch, scanned, h->tile_off2);
   CKLAUNCH("k_fused_offsets");
   ScatterParams<T> sp{};  // the ranking reads the cell words and the tables only
   sp.mx = f.mx;
@@ -628,9 +648,7 @@ int do_fused_sort(pbpic_handle* h) {
     CKLAUNCH("k_fused_perm");
     h->lazy = true;
   }
-  k_tile_off<<<grid_for(h->ntiles + 1, 256, 1 << 20), 256, 0, s>>>(h->off, h->ntiles, h->tpc, h->TY, h->cfg.my,
-                                                                  (int32_t)n, h->tile_off);
-  CKLAUNCH("k_tile_off");
+  std::swap(h->tile_off, h->tile_off2);
   h->sorted = true;
   h->hist_valid = false;
   return PBPIC_OK;
@@ -652,31 +670,42 @@ FilterParams<T> filter_params(pbpic_handle* h) {
   return f;
 }
 
+// The field solve; `ke`: the push's kinetic energies go into the same energy row.
 template <class T, bool MIXED>
-int do_fieldsolve(pbpic_handle* h) {
+int do_fieldsolve(pbpic_handle* h, bool ke = false) {
+  using Acc = typename std::conditional<MIXED, long long, double>::type;
   cudaStream_t s = h->stream;
+  TRY(ensure_hist(h, h->itime + 2));
   FieldParams<T> a = field_params<T, MIXED>(h);
+  if (!h->filters) {
+    a.jnext = h->jacc2;
+    a.ke_part = ke ? h->ke_part : nullptr;
+    a.nke = h->ntiles;
+    a.fe_scale = fe_scale(h->cfg);
+    a.fb_scale = fb_scale(h->cfg);
+    a.row = h->hist + (size_t)(h->itime + 1) * 4;
+    k_field_step<T, Acc><<<field_tiles(h->cfg.mx, h->cfg.my), FT, 0, s>>>(a);
+    CKLAUNCH("k_field_step");
+    for (int k = 0; k < 6; ++k) std::swap(h->f[k], h->f2[k]);
+    h->j2_clear = true;
+    h->itime += 1;
+    return PBPIC_OK;
+  }
   const int rows = h->cfg.ybc == 0 ? h->cfg.my : h->cfg.my + 1;
   const int g = grid_for((int64_t)h->cfg.mx * rows, 256);
   FilterParams<T> fp = filter_params<T, MIXED>(h);
   const int gf = grid_for((int64_t)h->cfg.mx * h->cfg.my, 256);
-  if (h->filters) {
-    if (MIXED) k_filter_prep<T, long long><<<gf, 256, 0, s>>>(a, fp);
-    else k_filter_prep<T, double><<<gf, 256, 0, s>>>(a, fp);
-    CKLAUNCH("k_filter_prep");
-  }
+  k_filter_prep<T, Acc><<<gf, 256, 0, s>>>(a, fp);
+  CKLAUNCH("k_filter_prep");
   k_bhalf<T><<<g, 256, 0, s>>>(a);
   CKLAUNCH("k_bhalf");
-  if (MIXED) k_efull<T, long long><<<g, 256, 0, s>>>(a);
-  else k_efull<T, double><<<g, 256, 0, s>>>(a);
+  k_efull<T, Acc><<<g, 256, 0, s>>>(a);
   CKLAUNCH("k_efull");
-  if (h->filters) {
-    k_filter_apply<T><<<gf, 256, 0, s>>>(a, fp);
-    CKLAUNCH("k_filter_apply");
-  }
+  k_filter_apply<T><<<gf, 256, 0, s>>>(a, fp);
+  CKLAUNCH("k_filter_apply");
   k_bhalf<T><<<g, 256, 0, s>>>(a);
   CKLAUNCH("k_bhalf");
-  TRY(nodes_and_field_energy<T, MIXED>(h, h->itime + 1));
+  TRY((nodes_and_field_energy<T, MIXED>(h, h->itime + 1, ke)));
   h->itime += 1;
   return PBPIC_OK;
 }
@@ -698,7 +727,7 @@ int do_step(pbpic_handle* h, int nsteps, int sort_every) {
     TRY(rp);
     const bool due = autosort || (sort_every > 0 && (h->itime + 1) % sort_every == 0);
     if (!(due && h->hist_valid)) {
-      TRY((do_fieldsolve<T, MIXED>(h)));
+      TRY((do_fieldsolve<T, MIXED>(h, true)));
       if (sort_every > 0 && h->itime % sort_every == 0) TRY((do_sort<T, MIXED>(h)));
       continue;
     }
@@ -711,7 +740,7 @@ int do_step(pbpic_handle* h, int nsteps, int sort_every) {
     CK(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
     const cudaStream_t main = h->stream;
     h->stream = h->side;
-    const int rf = do_fieldsolve<T, MIXED>(h);
+    const int rf = do_fieldsolve<T, MIXED>(h, true);
     h->stream = main;
     const int rs = rf == PBPIC_OK ? do_fused_sort<T, MIXED>(h) : rf;
     CK(cudaEventRecord(h->ev_join, h->side));  // joined on the error paths too
@@ -1031,12 +1060,16 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
     A(&h->vals[b], capn * 4);
   }
   for (int k = 0; k < 6; ++k) A(&h->f[k], (size_t)pe * h->tsz);
+  for (int k = 0; k < 6; ++k) A(&h->f2[k], (size_t)pe * h->tsz);
   A(&h->ng, (size_t)(c.mx + 1) * (c.my + 1) * 8 * h->tsz);
   if (h->mixed) A(&h->cg, (size_t)c.mx * c.my * 24 * h->tsz);
   A(&h->jacc, (size_t)4 * pe * 8);
+  A(&h->jacc2, (size_t)4 * pe * 8);
+  A(&h->ticket, 16);
   A(&h->counts, (size_t)(h->ncells + 1) * 4);
   A(&h->off, (size_t)(h->ncells + 1) * 4);
   A(&h->tile_off, (size_t)(h->ntiles + 1) * 4);
+  A(&h->tile_off2, (size_t)(h->ntiles + 1) * 4);
   A(&h->tilecnt, (size_t)h->ntiles * h->nb * 4);
   A(&h->tbase, (size_t)h->ntiles * h->nb * 4);
   A(&h->ke_part, (size_t)std::max(h->ntiles, 148 * 16) * 2 * 8);
@@ -1044,10 +1077,13 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
   h->bin_cap = (int64_t)h->ntiles * h->nb;
   h->nke = 148 * 8;
   h->nfe = grid_for((int64_t)(c.mx + 1) * (c.my + 1), 256, 148 * 8);
-  A(&h->fe_part, (size_t)h->nfe * 2 * 8);
+  A(&h->fe_part, (size_t)std::max(h->nfe, field_tiles(c.mx, c.my)) * 2 * 8);
   A(&h->status, 16);
   A(&h->rhist, (size_t)radix_hist_ints((int64_t)capn) * 4);
-  const int64_t sc = std::max(scan_scratch_ints(radix_hist_ints((int64_t)capn)), scan_scratch_ints(h->ncells + 1));
+  // (the fused sort's chunk totals and, beyond CS_MAXCHUNKS of them, the levels of their scan)
+  const int64_t nchunks = ((int64_t)h->ncells + 1 + CS_TILE - 1) / CS_TILE;
+  const int64_t sc = std::max({scan_scratch_ints(radix_hist_ints((int64_t)capn)), scan_scratch_ints(h->ncells + 1),
+                               nchunks + 1 + scan_scratch_ints(nchunks)});
   A(&h->scan_scratch, (size_t)sc * 4);
   A(&h->rho, (size_t)pe * 8);
   A(&h->dscalar, 64);  // scalars of the diagnostics (up to 4 doubles)
@@ -1062,6 +1098,7 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
   cudaMemset(h->counts, 0, (size_t)(h->ncells + 1) * 4);
   cudaMemset(h->off, 0, (size_t)(h->ncells + 1) * 4);
   cudaMemset(h->status, 0, 16);
+  cudaMemset(h->ticket, 0, 16);
   if (ensure_hist(h, 64) != PBPIC_OK || set_unsorted_tiles(h) != PBPIC_OK) {
     pbpic_destroy(h);
     return PBPIC_ENOMEM;
@@ -1554,7 +1591,7 @@ struct pbpic_batch {
   int ncells_tiles = 0, cells_blocks = 0;  // the table's first tiles: those pushed cell by cell
   bool track = false;                      // some domain carries particle ids
   size_t push_smem = 0, cells_smem = 0;
-  int gx_zero = 1, gx_cells = 1, gx_bins = 1, gx_tiles = 1, gx_field = 1, gx_nodes = 1;
+  int gx_zero = 1, gx_cells = 1, gx_tiles = 1, gx_field = 1, gx_nodes = 1;
 };
 
 namespace {
@@ -1587,10 +1624,12 @@ int retile(pbpic_handle* h, int ty) {
   CK(cudaStreamSynchronize(h->stream));
   if (ntiles > h->tile_cap) {
     dfree(h, h->tile_off);
+    dfree(h, h->tile_off2);
     dfree(h, h->ke_part);
-    h->tile_off = nullptr;
+    h->tile_off = h->tile_off2 = nullptr;
     h->ke_part = nullptr;
     TRY(dalloc(h, &h->tile_off, (size_t)(ntiles + 1) * 4));
+    TRY(dalloc(h, &h->tile_off2, (size_t)(ntiles + 1) * 4));
     TRY(dalloc(h, &h->ke_part, (size_t)std::max(ntiles, 148 * 16) * 2 * 8));
     h->tile_cap = ntiles;
   }
@@ -1643,8 +1682,8 @@ int batch_layout(pbpic_batch* b) {
   std::vector<Item> items;
   size_t smem = 0, csmem = 0;
   bool track = false;
-  int64_t maxcells = 1, maxbins = 1, maxtiles = 1, maxfield = 1, maxacc = 1;
-  int maxnfe = 1;
+  int64_t maxcells = 1, maxtiles = 1, maxfield = 1, maxacc = 1;
+  int maxnodes = 1;
   for (int d = 0; d < D; ++d) {
     const pbpic_handle* h = b->dom[d];
     const double ppc = (double)h->n / (double)h->ncells;
@@ -1657,12 +1696,10 @@ int batch_layout(pbpic_batch* b) {
     csmem = std::max(csmem, cells_smem_bytes(h->TY, true));
     track |= h->cfg.track_pid != 0;
     maxcells = std::max<int64_t>(maxcells, (int64_t)h->ncells + 1);
-    maxbins = std::max<int64_t>(maxbins, (int64_t)h->ntiles * h->nb);
     maxtiles = std::max<int64_t>(maxtiles, (int64_t)h->ntiles + 1);
-    const int rows = h->cfg.ybc == 0 ? h->cfg.my : h->cfg.my + 1;
-    maxfield = std::max<int64_t>(maxfield, (int64_t)h->cfg.mx * rows);
+    maxfield = std::max<int64_t>(maxfield, plane_elems(h));
+    maxnodes = std::max(maxnodes, field_tiles(h->cfg.mx, h->cfg.my));
     maxacc = std::max<int64_t>(maxacc, 2 * plane_elems(h));  // 16-byte stores of 4 planes
-    maxnfe = std::max(maxnfe, h->nfe);
   }
   std::stable_sort(items.begin(), items.end(), [](const Item& x, const Item& y) { return x.cells != y.cells ? x.cells : x.cost > y.cost; });
   if (items.size() > (size_t)0x7fffffff) return fail(PBPIC_EINVAL, "too many tiles in the batch");
@@ -1697,10 +1734,9 @@ int batch_layout(pbpic_batch* b) {
   b->scatter_blocks = std::max(1, std::min(b->ntiles, sms * std::max(1, per_sm)));
   b->gx_zero = grid_for(maxacc, 256, 1024);
   b->gx_cells = grid_for(maxcells, 256);
-  b->gx_bins = grid_for(maxbins, 256);
   b->gx_tiles = grid_for(maxtiles, 256, 1 << 16);
   b->gx_field = grid_for(maxfield, 256);
-  b->gx_nodes = maxnfe;
+  b->gx_nodes = maxnodes;
   (void)D;
   return PBPIC_OK;
 }
@@ -1756,7 +1792,6 @@ int batch_descriptors(pbpic_batch* b) {
     f.off = h->off;
     f.base = h->tbase;
     b->h_field[d] = field_params<float, true>(h);
-    b->h_field[d].nblk = h->nfe;
     TileOffDesc& t = b->h_toff[d];
     t.off = h->off;
     t.ntiles = h->ntiles;
@@ -1775,7 +1810,7 @@ int batch_descriptors(pbpic_batch* b) {
     e.ke_part = h->ke_part;
     e.nke = h->ntiles;
     e.fe_part = h->fe_part;
-    e.nfe = h->nfe;
+    e.nfe = field_tiles(h->cfg.mx, h->cfg.my);
     e.fe_scale = fe_scale(h->cfg);
     e.fb_scale = fb_scale(h->cfg);
     e.rows = h->hist + (size_t)(h->itime + 1) * 4;
@@ -1816,7 +1851,7 @@ int batch_enqueue_step(pbpic_batch* b, int par) {
   CKLAUNCH("k_fused_counts_batched");
   k_scan_batched<<<D, SCB, 0, s>>>(b->d_dom);
   CKLAUNCH("k_scan_batched");
-  k_fused_base_batched<<<dim3(b->gx_bins, D), 256, 0, s>>>(b->d_fsort);
+  k_fused_base_batched<<<dim3(b->gx_cells, D), 256, 0, s>>>(b->d_fsort);
   CKLAUNCH("k_fused_base_batched");
   k_fused_perm_batched<float><<<b->scatter_blocks, 256, 0, s>>>(b->d_scat + (size_t)par * D, b->d_tiles,
                                                                 b->ntiles, ctr + 1);
@@ -1831,7 +1866,7 @@ int batch_enqueue_step(pbpic_batch* b, int par) {
   CKLAUNCH("k_bhalf_batched");
   k_nodes_batched<float><<<dim3(b->gx_nodes, D), 256, 0, s>>>(b->d_field);
   CKLAUNCH("k_nodes_batched");
-  k_cell_records_batched<<<dim3(b->gx_nodes, D), 256, 0, s>>>(b->d_field);
+  k_cell_records_batched<<<dim3(grid_for(b->gx_field * 256, 256), D), 256, 0, s>>>(b->d_field);
   CKLAUNCH("k_cell_records_batched");
   k_energy_rows_batched<<<D, 256, 0, s>>>(b->d_erow, ctr + 2);
   CKLAUNCH("k_energy_rows_batched");

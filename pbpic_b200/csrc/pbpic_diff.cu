@@ -164,7 +164,7 @@ PushParams<T> push_params(const pbpic_diff* d, const Slot& s) {
 template <class T>
 FieldParams<T> field_params(const pbpic_diff* d, const Slot& s) {
   View<T> v = view<T>(d, s);
-  FieldParams<T> a;
+  FieldParams<T> a{};
   a.mx = d->mx;
   a.my = d->my;
   a.S = d->S;
