@@ -147,20 +147,6 @@ __device__ __forceinline__ void put_part(const Comps<T>& c, int64_t e, const P5<
   put_quad(c, e, p.dx, p.dy, p.ux, p.uy);
   c.z[e] = p.uz;
 }
-// One array a component (the differentiable form's states).
-template <class T>
-struct Soa5 {
-  T* c[5];
-};
-template <class T>
-__device__ __forceinline__ void put_part(const Soa5<T>& s, int64_t e, const P5<T>& p) {
-  s.c[0][e] = p.dx;
-  s.c[1][e] = p.dy;
-  s.c[2][e] = p.ux;
-  s.c[3][e] = p.uy;
-  s.c[4][e] = p.uz;
-}
-
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 __device__ __forceinline__ unsigned lanemask_lt() {
   unsigned m;

@@ -36,7 +36,7 @@ struct FieldParams {
   const double* ke_part; // kinetic partials of the push, or null
   int nke;
   double fe_scale, fb_scale;
-  double* row;           // null: no row (batched domains)
+  double* row;           // null: no energy row
   int* ticket;           // blocks finished so far (0 between launches)
 };
 
@@ -590,7 +590,7 @@ __device__ __forceinline__ void field_step_tile(const FieldParams<T>& a, int bid
     a.fe_part[2 * bid + 1] = tb;
   }
   if constexpr (sizeof(T) == 4) {
-    for (int e = threadIdx.x; e < FX * FY; e += FT) {
+    for (int e = threadIdx.x; a.cg && e < FX * FY; e += FT) {
       const int cx = i0 + e / FY, cy = j0 + e % FY;
       if (cx >= a.mx || cy >= a.my) continue;
       const int n = (e / FY) * FNY + e % FY;
@@ -608,6 +608,7 @@ template <class T, class Acc>
 __global__ void __launch_bounds__(FT) k_field_step(FieldParams<T> a) {
   __shared__ FieldTile<T> s;
   field_step_tile<T, Acc>(a, blockIdx.x, s);
+  if (!a.row) return;
   // the last block to finish adds up every block's partials, in the order of k_energy_row
   __threadfence();
   __syncthreads();

@@ -7,8 +7,8 @@ namespace pbd {
 
 // Device plasma loader: one thread per (ion, electron) pair, the same
 // generator and arithmetic as the host loader in pic_common.h.
-template <class T, class Arrays>
-__global__ void k_load(pic::LoadParams L, int64_t npairs, int electrons_only, uint32_t* cell, Arrays c,
+template <class T>
+__global__ void k_load(pic::LoadParams L, int64_t npairs, int electrons_only, uint32_t* cell, Comps<T> c,
                        int32_t* pid) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= npairs) return;

@@ -47,8 +47,9 @@ int grid_of(int64_t n, int maxblocks = 148 * 8) {
 
 // One stored state: particles and Yee fields.
 struct Slot {
-  void* p = nullptr;  // cell (4 B) then 5 component arrays of T
-  void* f = nullptr;  // 6 planes of T
+  void* p = nullptr;   // records of 4 T and uz (T), cell words, ids and permutation (4 B each)
+  void* f = nullptr;   // 6 planes of T
+  void* ng = nullptr;  // node grid of those fields
 };
 
 }  // namespace
@@ -63,16 +64,17 @@ struct pbpic_diff {
   int nseg = 0;
   std::vector<Slot> ck;   // checkpoints: state at steps 0, K, 2K, ...
   std::vector<Slot> seg;  // recomputed states of one segment (K + 1)
-  Slot work;              // running state
-  void* ng = nullptr;     // node grid of T
-  void* jacc = nullptr;   // 4 planes of 8-byte accumulators
+  Slot work[2];           // running states of a forward run
+  void* jacc[2] = {nullptr, nullptr};  // 4 planes of 8-byte accumulators; [0] is clear before a push
   double* fe_part = nullptr;
   int nfe = 0;
-  void* lam[2][5] = {{nullptr}};
+  int32_t *rank = nullptr, *counts = nullptr, *off = nullptr, *sums = nullptr;  // cell order of a new state
+  bool last_seg = false;  // seg holds the states of the forward run's last segment
+  void* lam[2] = {nullptr, nullptr};  // particle adjoints: records of 4 T, then uz
   double* fbar = nullptr;  // 6 adjoint planes (ex ey ez bx by bz)
   double* jbar = nullptr;  // 3 planes
   double* gbar = nullptr;  // node adjoint
-  double* scal = nullptr;  // [0] loss, [1] d loss / d omega, [2] d loss / d tau
+  double* scal = nullptr;  // [0] loss, [1] d loss / d omega, [2] d loss / d tau, [3] d loss / d psi0
   void* jseg = nullptr;    // j.E loss: the current of each step of the recomputed segment (3 planes each)
   pbpic_diff_params last{};
   bool have_forward = false;
@@ -89,23 +91,25 @@ int dmalloc(pbpic_diff* d, void** p, size_t bytes) {
   return PBPIC_OK;
 }
 
-size_t part_bytes(const pbpic_diff* d) { return (size_t)d->n * (4 + 5 * d->tsz); }
+size_t part_bytes(const pbpic_diff* d) { return (size_t)d->n * (12 + 5 * d->tsz); }
 size_t field_bytes(const pbpic_diff* d) { return (size_t)6 * d->mx * d->S * d->tsz; }
+size_t node_bytes(const pbpic_diff* d) { return (size_t)(d->mx + 1) * (d->my + 1) * 8 * d->tsz; }
 int64_t plane(const pbpic_diff* d) { return (int64_t)d->mx * d->S; }
 
 template <class T>
 struct View {
-  uint32_t* cell;
-  T* c[5];
+  DiffState<T> p;
   T* f[6];
 };
 
 template <class T>
 View<T> view(const pbpic_diff* d, const Slot& s) {
   View<T> v;
-  v.cell = (uint32_t*)s.p;
-  T* base = (T*)((char*)s.p + (size_t)d->n * 4);
-  for (int k = 0; k < 5; ++k) v.c[k] = base + (size_t)k * d->n;
+  T* base = (T*)s.p;
+  v.p.c = Comps<T>{base, base + (size_t)4 * d->n};
+  v.p.cell = (uint32_t*)(base + (size_t)5 * d->n);
+  v.p.id = (int32_t*)(v.p.cell + d->n);
+  v.p.perm = v.p.id + d->n;
   for (int k = 0; k < 6; ++k) v.f[k] = (T*)s.f + (size_t)k * plane(d);
   return v;
 }
@@ -131,7 +135,6 @@ double durel(double v) { return 1.0 / pow(1.0 - v * v, 1.5); }
 
 template <class T>
 PushParams<T> push_params(const pbpic_diff* d, const Slot& s) {
-  View<T> v = view<T>(d, s);
   PushParams<T> p;
   memset(&p, 0, sizeof(p));
   p.mx = d->mx;
@@ -139,10 +142,9 @@ PushParams<T> push_params(const pbpic_diff* d, const Slot& s) {
   p.S = d->S;
   p.ybc = PBPIC_BC_CONDUCTING;
   p.compat = 0;
-  p.cell = v.cell;
-  p.ng = (const T*)d->ng;
+  p.ng = (const T*)s.ng;
   p.cg = nullptr;  // the adjoint kernels gather from the node grid
-  p.jacc = d->jacc;
+  p.jacc = d->jacc[0];
   const T dt = (T)d->dt, mime = (T)d->cfg.mime, cva = (T)d->cva, dx = (T)d->dx, dy = (T)d->dy;
   for (int sp = 0; sp < 2; ++sp) {
     const T q = sp == 0 ? T(1) : T(-1);
@@ -180,9 +182,9 @@ FieldParams<T> field_params(const pbpic_diff* d, const Slot& s) {
   a.cdt = dt * (cva * cva);
   a.idx = T(1) / (T)d->dx;
   a.idy = T(1) / (T)d->dy;
-  a.jacc = d->jacc;
+  a.jacc = d->jacc[0];
   for (int k = 0; k < 4; ++k) a.jscale[k] = d->f32 ? d->in0 * FIX_INV : d->in0;
-  a.ng = (T*)d->ng;
+  a.ng = (T*)s.ng;
   a.cg = nullptr;
   a.fe_part = d->fe_part;
   return a;
@@ -221,49 +223,77 @@ int nodes(pbpic_diff* d, const Slot& s) {
   return PBPIC_OK;
 }
 
-// One forward step of a slot in place; adds the step's loss to scal[0]. With
+// Permutation into cell order of a state whose elements' ranks and cell counts are in
+// d->rank and d->counts; leaves the counts clear.
+int cell_offsets(pbpic_diff* d) {
+  const int64_t nc = (int64_t)d->mx * d->my;
+  const unsigned nb = (unsigned)((nc + CS_TILE - 1) / CS_TILE);
+  k_diff_scan<<<nb, CS_BT>>>(d->counts, nc, d->off, d->sums);
+  DLAUNCH("k_diff_scan");
+  k_diff_offsets<<<nb, CS_BT>>>(d->off, d->sums, nc);
+  DLAUNCH("k_diff_offsets");
+  return PBPIC_OK;
+}
+
+// One forward step from slot s to slot o; adds the step's loss to scal[0]. With
 // the j.E loss and `jkeep`, also keeps the step's current (3 planes) there.
 template <class T>
-int step(pbpic_diff* d, const Slot& s, double omega, void* jkeep = nullptr) {
-  DTRY(nodes<T>(d, s));
-  DCK(cudaMemsetAsync(d->jacc, 0, (size_t)4 * plane(d) * 8));
+int step(pbpic_diff* d, const Slot& s, const Slot& o, double omega, void* jkeep = nullptr) {
+  View<T> vs = view<T>(d, s), vo = view<T>(d, o);
   DiffParams<T> dp;
   memset(&dp, 0, sizeof(dp));
   dp.push = push_params<T>(d, s);
-  for (int k = 0; k < 5; ++k) dp.s[k] = view<T>(d, s).c[k];
   dp.n = d->n;
   dp.nsheet = d->nsheet;
   dp.omega_bg = omega;
   dp.in0 = d->in0;
-  k_dpush<T><<<grid_of(d->n, 148 * 16), 256>>>(dp);
+  dp.in = vs.p;
+  dp.out = vo.p;
+  dp.rank = d->rank;
+  dp.counts = d->counts;
+  k_dpush<T><<<(unsigned)((d->n + DT - 1) / DT), DT>>>(dp);
   DLAUNCH("k_dpush");
+  DTRY(cell_offsets(d));
+  k_diff_perm<<<grid_of(d->n, 148 * 16), 256>>>(vo.p.cell, d->rank, d->off, d->n, d->my, vo.p.perm);
+  DLAUNCH("k_diff_perm");
   const bool jdote = d->cfg.loss == PBPIC_LOSS_JDOTE;
   if (jdote) {
-    DTRY(loss_jdote<T>(d, s, d->jacc, d->scal, nullptr, nullptr));
-    if (jkeep) DCK(cudaMemcpyAsync(jkeep, d->jacc, (size_t)3 * plane(d) * 8, cudaMemcpyDeviceToDevice));
+    DTRY(loss_jdote<T>(d, s, d->jacc[0], d->scal, nullptr, nullptr));
+    if (jkeep) DCK(cudaMemcpyAsync(jkeep, d->jacc[0], (size_t)3 * plane(d) * 8, cudaMemcpyDeviceToDevice));
   }
   FieldParams<T> a = field_params<T>(d, s);
-  const int g = grid_of((int64_t)d->mx * (d->my + 1));
-  k_bhalf<T><<<g, 256>>>(a);
-  DLAUNCH("k_bhalf");
-  if (d->f32) k_efull<T, long long><<<g, 256>>>(a);
-  else k_efull<T, double><<<g, 256>>>(a);
-  DLAUNCH("k_efull");
-  k_bhalf<T><<<g, 256>>>(a);
-  DLAUNCH("k_bhalf");
-  DTRY(nodes<T>(d, s));
+  a.nex = vo.f[0];
+  a.ney = vo.f[1];
+  a.nez = vo.f[2];
+  a.nbx = vo.f[3];
+  a.nby = vo.f[4];
+  a.nbz = vo.f[5];
+  a.ng = (T*)o.ng;
+  a.jnext = d->jacc[1];
+  if (d->f32) k_field_step<T, long long><<<field_tiles(d->mx, d->my), FT>>>(a);
+  else k_field_step<T, double><<<field_tiles(d->mx, d->my), FT>>>(a);
+  DLAUNCH("k_field_step");
+  std::swap(d->jacc[0], d->jacc[1]);
   if (!jdote) {
-    k_loss_b<T><<<grid_of((int64_t)(d->mx + 1) * (d->my + 1)), 256>>>(d->mx, d->my, 1, (const T*)d->ng,
+    k_loss_b<T><<<grid_of((int64_t)(d->mx + 1) * (d->my + 1)), 256>>>(d->mx, d->my, 1, (const T*)o.ng,
                                                                        loss_scale(d), d->scal, nullptr);
     DLAUNCH("k_loss_b");
   }
   return PBPIC_OK;
 }
 
-int copy_slot(pbpic_diff* d, const Slot& dst, const Slot& src) {
-  DCK(cudaMemcpyAsync(dst.p, src.p, part_bytes(d), cudaMemcpyDeviceToDevice));
-  DCK(cudaMemcpyAsync(dst.f, src.f, field_bytes(d), cudaMemcpyDeviceToDevice));
-  return PBPIC_OK;
+pic::FieldInit field_init(const pbpic_diff* d, double psi0) {
+  pic::FieldInit f;
+  f.kind = pic::LOAD_HARRIS;
+  f.mx = d->mx;
+  f.my = d->my;
+  f.dx = d->dx;
+  f.dy = d->dy;
+  f.lambda = d->cfg.lambda;
+  f.psi0 = psi0;
+  f.bguide = 0.0;
+  f.b0z = 0.0;
+  return f;
 }
 
 template <class T>
@@ -287,44 +317,43 @@ int load(pbpic_diff* d, const pbpic_diff_params* prm) {
   L.udrift_i = urel(hs.udi);
   L.lambda = c.lambda;
   L.seed = c.seed;
-  View<T> v = view<T>(d, d->work);
-  k_load<T><<<(unsigned)((d->npairs + 255) / 256), 256>>>(L, d->npairs, 0, v.cell,
-                                                           Soa5<T>{{v.c[0], v.c[1], v.c[2], v.c[3], v.c[4]}}, nullptr);
+  // loaded in load order, then moved into cell order
+  View<T> v = view<T>(d, d->work[0]), v0 = view<T>(d, d->ck[0]);
+  k_load<T><<<(unsigned)((d->npairs + 255) / 256), 256>>>(L, d->npairs, 0, v.p.cell, v.p.c, nullptr);
   DLAUNCH("k_load");
-  pic::FieldInit fi;
-  fi.kind = pic::LOAD_HARRIS;
-  fi.mx = d->mx;
-  fi.my = d->my;
-  fi.dx = d->dx;
-  fi.dy = d->dy;
-  fi.lambda = c.lambda;
-  fi.psi0 = prm->psi0;
-  fi.bguide = 0.0;
-  fi.b0z = 0.0;
-  std::vector<T> yee((size_t)6 * plane(d), T(0));
-  for (int i = 0; i < d->mx; ++i)
-    for (int j = 0; j <= d->my; ++j) {
-      yee[(size_t)3 * plane(d) + (size_t)i * d->S + j] = (T)pic::init_bx(fi, i, j);
-      yee[(size_t)4 * plane(d) + (size_t)i * d->S + j] = (T)pic::init_by(fi, i, j);
-      yee[(size_t)5 * plane(d) + (size_t)i * d->S + j] = (T)pic::init_bz(fi, i, j);
-    }
-  DCK(cudaMemcpy(d->work.f, yee.data(), yee.size() * sizeof(T), cudaMemcpyHostToDevice));
-  return PBPIC_OK;
+  DCK(cudaMemsetAsync(d->counts, 0, (size_t)d->mx * d->my * 4));
+  DCK(cudaMemsetAsync(d->jacc[0], 0, (size_t)4 * plane(d) * 8));
+  k_diff_rank<<<(unsigned)((d->n + 255) / 256), 256>>>(v.p.cell, d->n, d->my, d->counts, d->rank);
+  DLAUNCH("k_diff_rank");
+  DTRY(cell_offsets(d));
+  k_diff_move<T><<<grid_of(d->n, 148 * 16), 256>>>(v.p.cell, v.p.c, d->rank, d->off, d->n, d->my, v0.p);
+  DLAUNCH("k_diff_move");
+  k_diff_fields<T><<<grid_of(plane(d)), 256>>>(field_init(d, prm->psi0), d->S, (T*)d->ck[0].f);
+  DLAUNCH("k_diff_fields");
+  return nodes<T>(d, d->ck[0]);
 }
 
 template <class T>
 int forward(pbpic_diff* d, const pbpic_diff_params* prm, double* loss) {
+  d->have_forward = d->last_seg = false;
   DTRY(load<T>(d, prm));
   DCK(cudaMemset(d->scal, 0, 4 * sizeof(double)));
   const int K = d->cfg.checkpoint_every, N = d->cfg.nsteps;
+  const int last0 = (d->nseg - 1) * K;  // first step of the last segment, whose states stay for the adjoint
   const double omega = prm->nb / d->cfg.nb0;
+  const size_t jbytes = (size_t)3 * plane(d) * 8;
+  // the state before step it: a checkpoint, a kept state of the last segment or a running state
+  auto slot = [&](int it) -> const Slot& {
+    if (it % K == 0 && it / K < d->nseg) return d->ck[it / K];
+    return it > last0 ? d->seg[it - last0] : d->work[it & 1];
+  };
   for (int it = 0; it < N; ++it) {
-    if (it % K == 0) DTRY(copy_slot(d, d->ck[it / K], d->work));
-    DTRY(step<T>(d, d->work, omega));
+    const bool keep = it >= last0 && d->jseg;
+    DTRY(step<T>(d, slot(it), slot(it + 1), omega, keep ? (char*)d->jseg + (it - last0) * jbytes : nullptr));
   }
   DCK(cudaMemcpy(loss, d->scal, sizeof(double), cudaMemcpyDeviceToHost));
   d->last = *prm;
-  d->have_forward = true;
+  d->have_forward = d->last_seg = true;
   return PBPIC_OK;
 }
 
@@ -360,30 +389,35 @@ int backward(pbpic_diff* d, double grad[3]) {
   const size_t nodes_bytes = (size_t)(d->mx + 1) * (d->my + 1) * 8 * sizeof(double);
   const bool jdote = d->cfg.loss == PBPIC_LOSS_JDOTE;
   const size_t jbytes = (size_t)3 * pl * 8;
-  for (int k = 0; k < 5; ++k) DCK(cudaMemset(d->lam[0][k], 0, (size_t)d->n * d->tsz));
+  DCK(cudaMemset(d->lam[0], 0, (size_t)5 * d->n * d->tsz));
+  auto lam = [&](int b) { return Comps<T>{(T*)d->lam[b], (T*)d->lam[b] + (size_t)4 * d->n}; };
   DCK(cudaMemset(d->fbar, 0, (size_t)6 * pl * sizeof(double)));
+  DCK(cudaMemset(d->gbar, 0, nodes_bytes));
   DCK(cudaMemset(d->scal + 1, 0, 3 * sizeof(double)));
   int cur = 0;
   AdjField af = adj_field(d);
   const int gf = grid_of((int64_t)d->mx * (d->my + 1));
   const int gn = grid_of((int64_t)(d->mx + 1) * (d->my + 1));
-  for (int sg = (N + K - 1) / K - 1; sg >= 0; --sg) {
+  // magnetic loss of a state: the seed of its node adjoint
+  auto seed = [&](const Slot& s) -> int {
+    k_loss_b<T><<<gn, 256>>>(d->mx, d->my, 1, (const T*)s.ng, loss_scale(d), nullptr, d->gbar);
+    DLAUNCH("k_loss_b");
+    return PBPIC_OK;
+  };
+  const bool resident = d->last_seg;
+  d->last_seg = false;  // (the segments before it are recomputed into its place)
+  for (int sg = d->nseg - 1; sg >= 0; --sg) {
     const int s0 = sg * K, s1 = std::min(N, s0 + K);
-    DTRY(copy_slot(d, d->seg[0], d->ck[sg]));
-    for (int m = 0; m < s1 - s0; ++m) {  // recompute the segment, keeping every state
-      DTRY(copy_slot(d, d->seg[m + 1], d->seg[m]));
-      DTRY(step<T>(d, d->seg[m + 1], omega, jdote ? (char*)d->jseg + m * jbytes : nullptr));
+    auto state = [&](int it) -> const Slot& { return it == s0 ? d->ck[sg] : d->seg[it - s0]; };
+    if (!(resident && sg == d->nseg - 1))
+      for (int it = s0; it < s1; ++it)  // recompute the segment, keeping every state
+        DTRY(step<T>(d, state(it), state(it + 1), omega, jdote ? (char*)d->jseg + (it - s0) * jbytes : nullptr));
+    if (sg == d->nseg - 1 && !jdote) {  // the last state's loss
+      DTRY(seed(state(N)));
+      k_adj_nodes<<<gn, 256>>>(af, d->gbar);
+      DLAUNCH("k_adj_nodes");
     }
     for (int it = s1 - 1; it >= s0; --it) {
-      const int m = it - s0;
-      if (!jdote) {  // magnetic loss of step it+1: seed the adjoint of the fields after the step
-        DTRY(nodes<T>(d, d->seg[m + 1]));
-        DCK(cudaMemsetAsync(d->gbar, 0, nodes_bytes));
-        k_loss_b<T><<<gn, 256>>>(d->mx, d->my, 1, (const T*)d->ng, loss_scale(d), nullptr, d->gbar);
-        DLAUNCH("k_loss_b");
-        k_adj_nodes<<<gn, 256>>>(af, d->gbar);
-        DLAUNCH("k_adj_nodes");
-      }
       // transposed field solve: B half step, E full step, B half step in reverse
       k_adj_bhalf<<<gf, 256>>>(af);
       DLAUNCH("k_adj_bhalf");
@@ -391,31 +425,33 @@ int backward(pbpic_diff* d, double grad[3]) {
       DLAUNCH("k_adj_efull");
       // j.E loss of step it: E (the step's start) into the current adjoint, the
       // step's current into the adjoint of that E
-      if (jdote) DTRY(loss_jdote<T>(d, d->seg[m], (char*)d->jseg + m * jbytes, nullptr, d->jbar, d->fbar));
-      k_zero_wall_ex<<<grid_of(d->mx), 256>>>(af);
-      DLAUNCH("k_zero_wall_ex");
+      if (jdote)
+        DTRY(loss_jdote<T>(d, state(it), (char*)d->jseg + (it - s0) * jbytes, nullptr, d->jbar, d->fbar));
       k_adj_bhalf<<<gf, 256>>>(af);
       DLAUNCH("k_adj_bhalf");
       // particle adjoint of the push of step it
-      DTRY(nodes<T>(d, d->seg[m]));
-      DCK(cudaMemsetAsync(d->gbar, 0, nodes_bytes));
       DiffParams<T> dp;
       memset(&dp, 0, sizeof(dp));
-      dp.push = push_params<T>(d, d->seg[m]);
-      for (int k = 0; k < 5; ++k) dp.s[k] = view<T>(d, d->seg[m]).c[k];
+      dp.push = push_params<T>(d, state(it));
       dp.n = d->n;
       dp.nsheet = d->nsheet;
       dp.omega_bg = omega;
       dp.in0 = d->in0;
-      for (int k = 0; k < 5; ++k) {
-        dp.lam_in[k] = (const T*)d->lam[cur][k];
-        dp.lam_out[k] = (T*)d->lam[1 - cur][k];
+      dp.in = view<T>(d, state(it)).p;
+      if (it == s1 - 1 && sg < d->nseg - 1) {  // lam comes in the order of the next checkpoint
+        k_diff_inverse<<<grid_of(d->n, 148 * 16), 256>>>(view<T>(d, d->ck[sg + 1]).p.id, d->n, d->rank);
+        DLAUNCH("k_diff_inverse");
+        dp.remap = d->rank;
       }
+      dp.lam_in = lam(cur);
+      dp.lam_out = lam(1 - cur);
       dp.jbar = d->jbar;
       dp.gbar = d->gbar;
       dp.domega = d->scal + 1;
-      k_dadjoint<T><<<grid_of(d->n, 148 * 16), 256>>>(dp);
+      k_dadjoint<T><<<(unsigned)((d->n + DT - 1) / DT), DT>>>(dp);
       DLAUNCH("k_dadjoint");
+      // the state's own magnetic loss (none at the start), in the same transposed node average
+      if (!jdote && it > 0) DTRY(seed(state(it)));
       k_adj_nodes<<<gn, 256>>>(af, d->gbar);
       DLAUNCH("k_adj_nodes");
       cur = 1 - cur;
@@ -431,35 +467,15 @@ int backward(pbpic_diff* d, double grad[3]) {
     const double dudi_v = du / ((1.0 + tite) * (1.0 + tite)), dude_v = du / ((1.0 + tite) * (1.0 + tite));
     View<T> v0 = view<T>(d, d->ck[0]);
     k_dtau<T><<<grid_of(d->n, 148 * 16), 256>>>(
-        d->n, d->nsheet, v0.c[2], v0.c[3], v0.c[4], (const T*)d->lam[cur][2], (const T*)d->lam[cur][3],
-        (const T*)d->lam[cur][4], urel(hs.vthi), urel(hs.vthe), durel(hs.vthi) * dvthi, durel(hs.vthe) * dvthe,
+        d->n, d->nsheet, v0.p.id, v0.p.c, lam(cur), urel(hs.vthi), urel(hs.vthe), durel(hs.vthi) * dvthi, durel(hs.vthe) * dvthe,
         urel(hs.udi), urel(hs.ude), durel(hs.udi) * dudi_v, durel(hs.ude) * dude_v, d->scal + 2);
     DLAUNCH("k_dtau");
   }
-  double sc[3];
-  DCK(cudaMemcpy(sc, d->scal + 1, 2 * sizeof(double), cudaMemcpyDeviceToHost));
-  // d loss / d psi0: the initial B is linear in psi0
-  std::vector<double> fb((size_t)2 * pl);
-  DCK(cudaMemcpy(fb.data(), d->fbar + 3 * pl, fb.size() * sizeof(double), cudaMemcpyDeviceToHost));
-  pic::FieldInit f1, f0;
-  f1.kind = f0.kind = pic::LOAD_HARRIS;
-  f1.mx = f0.mx = d->mx;
-  f1.my = f0.my = d->my;
-  f1.dx = f0.dx = d->dx;
-  f1.dy = f0.dy = d->dy;
-  f1.lambda = f0.lambda = d->cfg.lambda;
-  f1.bguide = f0.bguide = 0.0;
-  f1.b0z = f0.b0z = 0.0;
-  f1.psi0 = 1.0;
-  f0.psi0 = 0.0;
-  double gpsi = 0.0;
-  for (int i = 0; i < d->mx; ++i)
-    for (int j = 0; j <= d->my; ++j) {
-      const size_t o = (size_t)i * d->S + j;
-      gpsi += fb[o] * (pic::init_bx(f1, i, j) - pic::init_bx(f0, i, j));
-      if (j < d->my) gpsi += fb[pl + o] * (pic::init_by(f1, i, j) - pic::init_by(f0, i, j));
-    }
-  grad[0] = gpsi;
+  k_diff_psi<<<grid_of(pl), 256>>>(field_init(d, 0.0), d->S, d->fbar + 3 * pl, d->fbar + 4 * pl, d->scal + 3);
+  DLAUNCH("k_diff_psi");
+  double sc[3];  // d loss / d omega, d tau, d psi0
+  DCK(cudaMemcpy(sc, d->scal + 1, 3 * sizeof(double), cudaMemcpyDeviceToHost));
+  grad[0] = sc[2];
   grad[1] = sc[0] / d->cfg.nb0;
   grad[2] = sc[1];
   return PBPIC_OK;
@@ -504,22 +520,24 @@ int pbpic_diff_create(const pbpic_diff_config* cfg, pbpic_diff** out) {
   };
   d->ck.resize(d->nseg);
   d->seg.resize(c.checkpoint_every + 1);
-  for (auto& s : d->ck) {
+  auto slot = [&](Slot& s) {
     A(&s.p, part_bytes(d));
     A(&s.f, field_bytes(d));
-  }
-  for (auto& s : d->seg) {
-    A(&s.p, part_bytes(d));
-    A(&s.f, field_bytes(d));
-  }
-  A(&d->work.p, part_bytes(d));
-  A(&d->work.f, field_bytes(d));
-  A(&d->ng, (size_t)(c.mx + 1) * (c.my + 1) * 8 * d->tsz);
-  A(&d->jacc, (size_t)4 * plane(d) * 8);
+    A(&s.ng, node_bytes(d));
+  };
+  for (auto& s : d->ck) slot(s);
+  for (size_t k = 1; k < d->seg.size(); ++k) slot(d->seg[k]);  // (a segment's first state is its checkpoint)
+  slot(d->work[0]);
+  slot(d->work[1]);
+  for (int k = 0; k < 2; ++k) A(&d->jacc[k], (size_t)4 * plane(d) * 8);
+  const int64_t nc = (int64_t)c.mx * c.my;
+  A((void**)&d->rank, (size_t)d->n * 4);
+  A((void**)&d->counts, (size_t)nc * 4);
+  A((void**)&d->off, (size_t)nc * 4);
+  A((void**)&d->sums, (size_t)((nc + CS_TILE - 1) / CS_TILE + 1) * 4);
   d->nfe = grid_of((int64_t)(c.mx + 1) * (c.my + 1));
-  A((void**)&d->fe_part, (size_t)d->nfe * 2 * sizeof(double));
-  for (int b = 0; b < 2; ++b)
-    for (int k = 0; k < 5; ++k) A(&d->lam[b][k], (size_t)d->n * d->tsz);
+  A((void**)&d->fe_part, (size_t)std::max(d->nfe, field_tiles(c.mx, c.my)) * 2 * sizeof(double));
+  for (int b = 0; b < 2; ++b) A(&d->lam[b], (size_t)5 * d->n * d->tsz);
   A((void**)&d->fbar, (size_t)6 * plane(d) * sizeof(double));
   A((void**)&d->jbar, (size_t)3 * plane(d) * sizeof(double));
   A((void**)&d->gbar, (size_t)(c.mx + 1) * (c.my + 1) * 8 * sizeof(double));
