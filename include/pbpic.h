@@ -250,7 +250,10 @@ int pbpic_kernel_launches(int64_t* count);
 /* Stable counting sort of n cell keys in [0, ncells): perm[j] is the index of
  * the j-th key in sorted order and counts[c] the number of keys in cell c
  * (both device pointers). The same algorithm as pbpic_sort, exposed on raw
- * device buffers; allocates its scratch with cudaMalloc on each call.
+ * device buffers. Its scratch (at most 16 bytes a key) comes from a memory pool
+ * of the library's own, in the order of `stream`; up to 256 MB of it stay
+ * reserved per device for the next call, until a handle is destroyed or an
+ * allocation of the library fails.
  * stream is a cudaStream_t passed as void*. Replaces the ordering part of
  * countingsort (pic2d.f90:1303-1329). */
 int pbpic_counting_sort_keys(const int32_t* keys_dev, int64_t n, int32_t ncells,

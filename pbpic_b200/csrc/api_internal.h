@@ -6,3 +6,5 @@
 int pbpic_internal_fail(int code, const std::string& msg);
 // Count one kernel launch (reported by pbpic_kernel_launches).
 void pbpic_internal_count_launch();
+// Give back the device memory the library holds in reserve (before retrying an allocation).
+void pbpic_internal_trim();

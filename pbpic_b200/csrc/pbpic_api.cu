@@ -94,35 +94,86 @@ int scan_excl(cudaStream_t s, int32_t* data, int64_t n, int32_t* scratch) {
 }
 
 // ------------------------------------------------------------ radix sort
-int radix_passes(int32_t ncells) {
+int key_bits(int32_t ncells) {
   int bits = 1;
   while (bits < 31 && (1ll << bits) < (int64_t)ncells) ++bits;
-  return (bits + 7) / 8;
+  return bits;
+}
+int radix_passes(int32_t ncells) { return (key_bits(ncells) + RBITS - 1) / RBITS; }
+
+int64_t radix_hist_ints(int64_t n) { return RBINS * ((n + RTILE - 1) / RTILE); }
+
+// Stable LSD radix sort of keys[0..n) (values: the indices) into perm. The passes ping-pong
+// between (k1, v1) and (k0, v0); k0 may be the keys' own array, and v0 and v1 are not
+// needed for one pass, k0 and v0 not for two. perm is not the last pass's input (v0
+// for an odd number of passes above one, v1 for an even one).
+int radix_sort(cudaStream_t s, int64_t n, int32_t ncells, const int32_t* keys, int32_t* k0, int32_t* k1, int32_t* v0,
+               int32_t* v1, int32_t* rhist, int32_t* scan_scratch, int32_t* perm) {
+  const int total = key_bits(ncells), passes = radix_passes(ncells), bits = (total + passes - 1) / passes;
+  const int nblocks = (int)((n + RTILE - 1) / RTILE);
+  const int64_t nh = (int64_t)(1 << bits) * nblocks, nch = (nh + SCAN_TILE - 1) / SCAN_TILE;
+  const int32_t *kin = keys, *vin = nullptr;
+  for (int p = 0; p < passes; ++p) {
+    const bool last = p + 1 == passes;
+    int32_t* kout = last ? nullptr : (p & 1 ? k0 : k1);
+    int32_t* vout = last ? perm : (p & 1 ? v0 : v1);
+    k_radix_up<<<nblocks, RB, 0, s>>>(kin, n, bits * p, bits, rhist, nblocks);
+    CKLAUNCH("k_radix_up");
+    if (nch <= CS_MAXCHUNKS) {
+      k_scan_local<<<(unsigned)nch, SCAN_BT, 0, s>>>(rhist, rhist, nh, scan_scratch);
+      CKLAUNCH("k_scan_local");
+      if (nch > 1) {
+        k_scan_prefix<<<(unsigned)nch, SCAN_BT, 0, s>>>(rhist, nh, scan_scratch);
+        CKLAUNCH("k_scan_prefix");
+      }
+    } else {
+      TRY(scan_excl(s, rhist, nh, scan_scratch));
+    }
+    k_radix_down<<<nblocks, RB, 0, s>>>(kin, vin, n, bits * p, bits, rhist, nblocks, kout, vout);
+    CKLAUNCH("k_radix_down");
+    kin = kout;
+    vin = vout;
+  }
+  return PBPIC_OK;
 }
 
-int64_t radix_hist_ints(int64_t n) { return 256 * ((n + RTILE - 1) / RTILE); }
+// Scratch of the stateless sort: a memory pool of this library's own per device, of which up to
+// kSortKeep bytes stay reserved between calls (mapping 60 MB anew took three quarters of
+// a 5 M key sort). Allocations are ordered on the caller's stream, so calls on
+// several streams and threads share it safely. pbpic_destroy and a failed
+// device allocation give the reserve back.
+constexpr uint64_t kSortKeep = 256ull << 20;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pools[1024] = {};
 
-// Stable LSD radix sort of keys k0[0..n) (values: the indices). Buffers k0/k1
-// and v0/v1 ping-pong; returns the buffer holding the permutation.
-int radix_sort(cudaStream_t s, int64_t n, int32_t ncells, int32_t* k0, int32_t* k1, int32_t* v0,
-               int32_t* v1, int32_t* rhist, int32_t* scan_scratch, int32_t** perm) {
-  const int passes = radix_passes(ncells);
-  const int nblocks = (int)((n + RTILE - 1) / RTILE);
-  int32_t *kin = k0, *kout = k1, *vin = nullptr, *vout = v1;
-  int32_t* other_v = v0;
-  for (int p = 0; p < passes; ++p) {
-    k_radix_up<<<nblocks, RB, 0, s>>>(kin, n, 8 * p, rhist, nblocks);
-    CKLAUNCH("k_radix_up");
-    TRY(scan_excl(s, rhist, (int64_t)256 * nblocks, scan_scratch));
-    k_radix_down<<<nblocks, RB, 0, s>>>(kin, vin, n, 8 * p, rhist, nblocks, kout, vout);
-    CKLAUNCH("k_radix_down");
-    std::swap(kin, kout);
-    vin = vout;
-    vout = other_v;
-    other_v = vin;
+int sort_pool(cudaMemPool_t* out) {
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 1024) return fail(PBPIC_EINVAL, "device ordinal out of range");
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (!g_pools[dev]) {
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    CK(cudaMemPoolCreate(&p, &props));
+    uint64_t keep = kSortKeep;
+    CK(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
+    g_pools[dev] = p;
   }
-  *perm = vin;
+  *out = g_pools[dev];
   return PBPIC_OK;
+}
+
+// Gives back what the current device's pool holds and no call uses.
+void trim_sort_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 1024) return;
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (g_pools[dev]) cudaMemPoolTrimTo(g_pools[dev], 0);
 }
 
 template <class T>
@@ -133,6 +184,7 @@ struct DevT {
 }  // namespace
 
 int pbpic_internal_fail(int code, const std::string& msg) { return fail(code, msg); }
+void pbpic_internal_trim() { trim_sort_pool(); }
 void pbpic_internal_count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
 // ===================================================================== handle
@@ -211,6 +263,11 @@ namespace {
 int dalloc(pbpic_handle* h, void** p, size_t bytes) {
   if (bytes == 0) bytes = 16;
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    trim_sort_pool();
+    e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     *p = nullptr;
     return fail(PBPIC_ENOMEM, std::string("cudaMalloc(") + std::to_string(bytes) + "): " + cudaGetErrorString(e));
@@ -528,9 +585,10 @@ int do_sort(pbpic_handle* h) {
     }
   }
   if (n > 0 && !runs) {
-    int32_t* perm = nullptr;
-    TRY(radix_sort(s, n, h->ncells, h->keys[0], h->keys[1], h->vals[0], h->vals[1], h->rhist, h->scan_scratch,
-                   &perm));
+    const int np = radix_passes(h->ncells);
+    int32_t* perm = np > 1 && (np & 1) ? h->vals[1] : h->vals[0];
+    TRY(radix_sort(s, n, h->ncells, h->keys[0], h->keys[0], h->keys[1], h->vals[0], h->vals[1], h->rhist,
+                   h->scan_scratch, perm));
     k_gather<T><<<grid_for(n, 256), 256, 0, s>>>(perm, n, h->cell[b], C<T>(h, b), h->pid[b], h->cell[o], C<T>(h, o),
                                                   h->pid[o]);
     CKLAUNCH("k_gather");
@@ -1122,6 +1180,7 @@ int pbpic_destroy(pbpic_handle* h) {
   if (h->ev_join) cudaEventDestroy(h->ev_join);
   for (void* p : h->allocs) cudaFree(p);
   delete h;
+  trim_sort_pool();
   return PBPIC_OK;
 }
 
@@ -1413,16 +1472,22 @@ int pbpic_counting_sort_keys(const int32_t* keys_dev, int64_t n, int32_t ncells,
   if (!counts_dev) return fail(PBPIC_EINVAL, "null counts buffer");
   cudaStream_t s = (cudaStream_t)stream;
   const size_t nn = (size_t)std::max<int64_t>(n, 1);
+  const int passes = radix_passes(ncells);
+  // one pass reads the keys while it writes perm: overlapping buffers need a copy of the keys
+  const bool copy = passes == 1 && perm_dev < keys_dev + n && keys_dev < perm_dev + n;
+  const int pairs = copy ? 1 : (passes == 1 ? 0 : (passes == 2 ? 1 : 2));  // buffers of n keys and n values between passes
   const int64_t rh = radix_hist_ints((int64_t)nn);
   const int64_t sc = std::max(scan_scratch_ints(rh), (int64_t)16);
-  const size_t bytes = nn * 4 * 4 + (size_t)rh * 4 + (size_t)sc * 4 + 16;
+  const size_t bytes = nn * 8 * pairs + (size_t)rh * 4 + (size_t)sc * 4 + 16;
+  cudaMemPool_t pool = nullptr;
+  TRY(sort_pool(&pool));
   char* buf = nullptr;
-  CK(cudaMallocAsync((void**)&buf, bytes, s));
-  int32_t* k0 = (int32_t*)buf;
-  int32_t* k1 = k0 + nn;
-  int32_t* v0 = k1 + nn;
-  int32_t* v1 = v0 + nn;
-  int32_t* rhist = v1 + nn;
+  CK(cudaMallocFromPoolAsync((void**)&buf, bytes, pool, s));
+  int32_t* k1 = (int32_t*)buf;
+  int32_t* v1 = k1 + (pairs >= 1 ? nn : 0);
+  int32_t* k0 = v1 + (pairs >= 1 ? nn : 0);
+  int32_t* v0 = k0 + (pairs >= 2 ? nn : 0);
+  int32_t* rhist = v0 + (pairs >= 2 ? nn : 0);
   int32_t* scr = rhist + rh;
   int* status = (int*)(scr + sc);
   int rc = PBPIC_OK;
@@ -1440,17 +1505,11 @@ int pbpic_counting_sort_keys(const int32_t* keys_dev, int64_t n, int32_t ncells,
       rc = fail(PBPIC_ECUDA, "k_key_hist launch failed");
       break;
     }
-    if (cudaMemcpyAsync(k0, keys_dev, (size_t)n * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
+    if (copy && cudaMemcpyAsync(k1, keys_dev, (size_t)n * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
       rc = fail(PBPIC_ECUDA, "key copy failed");
       break;
     }
-    int32_t* perm = nullptr;
-    rc = radix_sort(s, n, ncells, k0, k1, v0, v1, rhist, scr, &perm);
-    if (rc != PBPIC_OK) break;
-    if (cudaMemcpyAsync(perm_dev, perm, (size_t)n * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
-      rc = fail(PBPIC_ECUDA, "permutation copy failed");
-      break;
-    }
+    rc = radix_sort(s, n, ncells, copy ? k1 : keys_dev, k0, k1, v0, v1, rhist, scr, perm_dev);
   } while (0);
   if (cudaMemcpyAsync(&st, status, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess && rc == PBPIC_OK)
     rc = fail(PBPIC_ECUDA, "status copy failed");
@@ -1484,7 +1543,7 @@ int pbpic_counting_sort_keys(const int32_t* keys_dev, int64_t n, int32_t ncells,
 namespace {
 
 constexpr int64_t kStaticKeys = PBPIC_STATIC_SORT_MAX_KEYS;
-constexpr int64_t kStaticHist = 256 * ((kStaticKeys + RTILE - 1) / RTILE);
+constexpr int64_t kStaticHist = RBINS * ((kStaticKeys + RTILE - 1) / RTILE);
 constexpr int64_t kStaticScan = 1024;  // chunk totals of every scan level of the histogram (needs 19)
 constexpr int64_t kStaticWords = 4 * kStaticKeys + kStaticHist + kStaticScan + 64;
 
@@ -1536,10 +1595,10 @@ extern "C" int pbpic_counting_sort_keys_static(const int32_t* keys_dev, int64_t 
   if (n > 0) {
     k_key_hist<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(keys_dev, n, ncells, counts_dev, status);
     CKLAUNCH("k_key_hist");
-    CK(cudaMemcpyAsync(k0, keys_dev, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
-    int32_t* perm = nullptr;
-    TRY(radix_sort(s, n, ncells, k0, k1, v0, v1, rhist, scr, &perm));
-    CK(cudaMemcpyAsync(perm_dev, perm, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
+    // (one pass reads the keys while it writes perm: overlapping buffers need a copy of the keys)
+    const bool copy = radix_passes(ncells) == 1 && perm_dev < keys_dev + n && keys_dev < perm_dev + n;
+    if (copy) CK(cudaMemcpyAsync(k1, keys_dev, (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
+    TRY(radix_sort(s, n, ncells, copy ? k1 : keys_dev, k0, k1, v0, v1, rhist, scr, perm_dev));
   }
   int st = 0;
   CK(cudaMemcpyAsync(&st, status, sizeof(int), cudaMemcpyDeviceToHost, s));

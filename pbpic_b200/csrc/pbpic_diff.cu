@@ -85,6 +85,11 @@ namespace {
 
 int dmalloc(pbpic_diff* d, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    pbpic_internal_trim();
+    e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+  }
   if (e != cudaSuccess)
     return pbpic_internal_fail(PBPIC_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   d->allocs.push_back(*p);
