@@ -671,4 +671,15 @@ static __global__ void k_cell_records_batched(const FieldParams<float>* d) {
   cell_records_body(a, blockIdx.x, gridDim.x);
 }
 
+// The accumulated current as the caller's array: component c times its scale. One pass here and
+// one copy; with the scaling and a second array on the host the read took 336 us at
+// 256x128 cells (1 MB), 258 us so.
+template <class A>
+__global__ void k_denjr(int64_t pe, const A* __restrict__ acc, double4 sc, double* __restrict__ out) {
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < 4 * pe; k += (int64_t)gridDim.x * blockDim.x) {
+    const double s = k < pe ? sc.x : (k < 2 * pe ? sc.y : (k < 3 * pe ? sc.z : sc.w));
+    out[k] = __dmul_rn((double)acc[k], s);
+  }
+}
+
 }  // namespace pbd

@@ -22,21 +22,25 @@
 // What bounds it, and why this form (512x256 Harris sheet, 26.2 M particles): the tile
 // push of kernels_push.cuh takes 575 us, 14.7 warp instructions a
 // particle at 65 % issue, a third of them moving registers, decoding cells and running
-// the crossers' branch for one or two lanes. This form takes 370 us with
-// 10.5 warp instructions a particle at 74 % issue: bound by instruction issue.
+// the crossers' branch for one or two lanes. This form takes 366 us with
+// 10.0 warp instructions a particle at 72 % issue: bound by instruction issue.
 // On the way there: particles loaded into registers one pass ahead, 540 us and 45 % of
 // the warps' time waiting for loads (the permutation entry, one pass
 // ahead, then the particle: two DRAM latencies in one pass's time); dx, dy, ux, uy as one
 // 16-byte record in place of four arrays, 450 us; the particles by asynchronous
 // copies, 435 us at any depth, because the permutation entries still came one
 // pass ahead; those through the ring too, 370 us. Blocks of 4 warps, 5 per SM at 96
-// registers (4 per SM: 385 us; 6 per SM spill: 500 us).
+// registers (4 per SM: 385 us; 6 per SM spill: 500 us). A species' constants come from a
+// table in shared memory, with zero charge and mass for lanes beyond the cell, and a
+// crosser is queued as one 16-byte record: 10.7 -> 10.0 instructions, step 453 -> 442 us.
+// Shared memory beyond this (buffers padded to a power of two: 207 KB an SM) takes the
+// L1 lines that the 4-byte copies share: 410 us.
 //
 // Plain form: the same with the coefficients read from shared memory in every pass (24 more
 // FP64 registers would cost a block per SM) and no window: a cell's 17 sums and
 // the crossers' 8 values go straight to the global current as reductions in L2 (FP64
 // atomics in shared memory are compare-and-swap loops, on which the crossers of one cell
-// collide). Its step on the same sheet: 1230 -> 763 us (the tile push 1041 us of it
+// collide). Its step on the same sheet: 1230 -> 703 us (the tile push 1041 us of it
 // before); 3 blocks per SM at 146 registers (4 at 128: 758 us, but 1.5 % slower at 128x128 cells).
 #pragma once
 #include "kernels_push.cuh"
@@ -118,8 +122,9 @@ __device__ __forceinline__ void end_group() { asm volatile("cp.async.commit_grou
 template <class T>
 struct CellsSmem {
   PassBuf<T> pass[PC_WARPS][PC_STAGES];
-  T q[PC_WARPS][4][PC_QUEUE];         // crossers: x, y before, x, y after the move
-  uint32_t qw[PC_WARPS][PC_QUEUE];    // and the old cell's word
+  alignas(16) T q[PC_WARPS][PC_QUEUE][4];  // crossers: x, y before, x, y after the move
+  int2 qw[PC_WARPS][PC_QUEUE];             // and the old cell's word, the position
+  alignas(16) T spc[3][8];                 // ion, electron, no particle: c0, c1, q, its mass as an electron, as an ion
   int32_t off[65];                 // positions of the tile's cells
   double red[32];
   uint64_t mbar;
@@ -134,6 +139,8 @@ struct CellsWin {
   int ixt, y0, mx, my, S, walls;
   double* jacc;
   double fx, fy;
+  uint32_t* cell;  // where the pushed particles go
+  void* quad;
 };
 
 __device__ __forceinline__ void shared_add(unsigned addr, unsigned v) {
@@ -168,19 +175,52 @@ __device__ __forceinline__ void deposit_at(const CellsWin& w, int c, int wx, int
 template <class T>
 __device__ __forceinline__ int cell_step(T x) { return x > T(0.5) ? 1 : (x < T(-0.5) ? -1 : 0); }
 
-// Empties `n` (<= 32) queued crossers, those at [first, first + n): both zig-zag
-// segments (pic2d.f90:1237-1272) to the window and the count from the old
-// cell's bin to the new one's.
-template <class T>
-__device__ __noinline__ void drain_crossers(const CellsWin w, const T* q, const uint32_t* qw, int first, int n) {
+__device__ __forceinline__ void get_quad(const float* p, float& a, float& b, float& c, float& d) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  a = v.x, b = v.y, c = v.z, d = v.w;
+}
+__device__ __forceinline__ void get_quad(const double* p, double& a, double& b, double& c, double& d) {
+  const double2 u = reinterpret_cast<const double2*>(p)[0], v = reinterpret_cast<const double2*>(p)[1];
+  a = u.x, b = u.y, c = v.x, d = v.y;
+}
+__device__ __forceinline__ void set_quad(float* p, float a, float b, float c, float d) {
+  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+__device__ __forceinline__ void set_quad(double* p, double a, double b, double c, double d) {
+  reinterpret_cast<double2*>(p)[0] = make_double2(a, b);
+  reinterpret_cast<double2*>(p)[1] = make_double2(c, d);
+}
+__device__ __forceinline__ void put_xy(float* p, float x, float y) { *reinterpret_cast<float2*>(p) = make_float2(x, y); }
+__device__ __forceinline__ void put_xy(double* p, double x, double y) { *reinterpret_cast<double2*>(p) = make_double2(x, y); }
+
+// Empties `n` (<= 32) queued crossers, those at [first, first + n): both zig-zag segments
+// (pic2d.f90:1237-1272) to the window, the count from the old cell's bin to the new
+// one's, and with RESOLVE the new cell and the offsets in it (kernels_push.cuh: push_core)
+// over what the pass stored. Returns the status bits.
+template <class T, bool RESOLVE>
+__device__ __noinline__ int drain_crossers(const CellsWin w, const T (*q)[4], const int2* qw, int first, int n) {
   const int lane = (int)lane_id();
+  int status = 0;
   __syncwarp();
   if (lane < n) {
     const int e = first + lane;
-    const T px = q[e], py = q[PC_QUEUE + e], x1 = q[2 * PC_QUEUE + e], y1 = q[3 * PC_QUEUE + e];
-    const uint32_t wrd = qw[e];
+    T px, py, x1, y1;
+    get_quad(q[e], px, py, x1, y1);
+    const int2 wp = qw[e];
+    const uint32_t wrd = (uint32_t)wp.x;
     const int iy = cw_iy(wrd), key = iy - w.y0, dcx = cell_step(x1), dcy = cell_step(y1);
+    if (M<T, true>::abs(x1) > T(1.5) || M<T, true>::abs(y1) > T(1.5)) status = PBPIC_STATUS_CELL_JUMP;
     const bool refl = w.walls && (unsigned)(iy + dcy) >= (unsigned)w.my;
+    if (RESOLVE) {
+      int nix = w.ixt + dcx, niy = refl ? iy : iy + dcy;
+      nix = nix < 0 ? nix + w.mx : (nix >= w.mx ? nix - w.mx : nix);
+      niy = niy < 0 ? niy + w.my : (niy >= w.my ? niy - w.my : niy);
+      T* out = static_cast<T*>(w.quad) + 4 * (int64_t)wp.y;
+      const T ny = M<T, true>::sub(y1, (T)dcy);
+      put_xy(out, M<T, true>::sub(x1, (T)dcx), refl ? -ny : ny);
+      if (refl) out[3] = -out[3];
+      w.cell[wp.y] = (wrd & 0x80000000u) | ((uint32_t)nix << 16) | (uint32_t)niy;
+    }
     const int row1 = refl ? key : key + dcy;  // a reflected particle keeps its row
     const T qq = (int)wrd < 0 ? T(-1) : T(1), half = T(0.5), one = T(1);
     using A = M<T, true>;
@@ -208,6 +248,7 @@ __device__ __noinline__ void drain_crossers(const CellsWin w, const T* q, const 
     }
   }
   __syncwarp();
+  return status;
 }
 
 // The 17 stencil entries (kernels_push.cuh: stencil_node) of the accumulated
@@ -279,6 +320,11 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
   using A = M<T, true>;
   constexpr bool F32 = sizeof(T) == 4;
   constexpr int GRP = 32 / L;
+  // Where a crosser's new cell is found: in the queue, whose 32 lanes are all crossers, or in the pass, where one
+  // or two lanes of 32 are. The first saves instructions (20 of 330 a pass) but writes a crosser twice. Step,
+  // queue against pass: 64x64 cells 36.0/37.3 us, 193x131 74.4/77.8, FP64 128x128 80.7/82.3, 512x256 703/708; but
+  // at 200 particles a cell, 512x256 FP32 455/444 us: there the extra writes cost more than the instructions.
+  constexpr bool LATE = L == 16 || !F32;
   const T half = T(0.5), one = T(1);
   CellsWin w;
   w.TY = a.tile_rows;
@@ -302,6 +348,8 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
   w.jacc = reinterpret_cast<double*>(a.jacc);
   w.fx = F32 ? 1.0 : (double)a.qx[0];
   w.fy = F32 ? 1.0 : (double)a.qy[0];
+  w.cell = GATHER ? a.cell_o : a.cell;
+  w.quad = GATHER ? a.c_o.q : a.c.q;
   if constexpr (F32) {
     if (threadIdx.x == 0) {  // the records of the tile's cells: one bulk copy
       const unsigned bytes = (unsigned)nrow * 96u;
@@ -320,16 +368,25 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
     const int by = e - (w.TY + 2);
     hist[e] = by >= 1 && by <= nrow ? a.cell_off[cell0 + by] - a.cell_off[cell0 + by - 1] : 0;
   }
+  if (threadIdx.x < 3) {
+    T* sp = sm.spc[threadIdx.x];
+    const int k = threadIdx.x;
+    sp[0] = k == 2 ? T(0) : a.c0[k & 1];
+    sp[1] = k == 2 ? T(0) : a.c1[k & 1];
+    sp[2] = k == 2 ? T(0) : (k == 1 ? T(-1) : one);
+    sp[3] = k == 1 ? a.ms[1] : T(0);
+    sp[4] = k == 0 ? a.ms[0] : T(0);
+  }
   __syncthreads();
   w.split = sm.off[nrow] - sm.off[0] <= 32767;
   const int plast = sm.off[nrow] - 1;
-  const bool edge = ixt == 0 || ixt == a.mx - 1 || y0 == 0 || y1 == a.my;  // a step may leave the domain
+  [[maybe_unused]] const bool edge = ixt == 0 || ixt == a.mx - 1 || y0 == 0 || y1 == a.my;  // a step may leave the domain
   bool staged = true;
   if constexpr (F32) staged = mbar_wait(&sm.mbar, parity);
   const int lane = (int)lane_id(), wp = threadIdx.x >> 5;
   const int grp = lane / L, gl = lane % L;
-  T* q = &sm.q[wp][0][0];
-  uint32_t* qw = sm.qw[wp];
+  T(*q)[4] = sm.q[wp];
+  int2* qw = sm.qw[wp];
   int nq = 0;
   // this lane's entry of the stencil once a group's sums are spread over its lanes (L = 32: a pair
   // of lanes holds the same sum, lane 1 takes the last entry)
@@ -385,7 +442,11 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
       start_elem<GATHER>(a, ring + 3, lane, take(ka));
       end_group();
     }
-    int slot = 0;
+    unsigned at = 0;  // the pass's buffer: a byte offset in the ring
+    constexpr unsigned STRIDE = sizeof(PassBuf<T>);
+    auto buf = [&](unsigned o) -> PassBuf<T>* {
+      return reinterpret_cast<PassBuf<T>*>(reinterpret_cast<unsigned char*>(ring) + o);
+    };
     T acc[17];
 #pragma unroll
     for (int k = 0; k < 17; ++k) acc[k] = T(0);
@@ -412,25 +473,19 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
         left -= chunk;
         do {
           asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-          const PassBuf<T>& in = ring[slot];
+          const PassBuf<T>& in = *buf(at);
           T quad[4];
-          if constexpr (F32) {
-            const float4 v = *reinterpret_cast<const float4*>(in.quad[lane]);
-            quad[0] = v.x, quad[1] = v.y, quad[2] = v.z, quad[3] = v.w;
-          } else {
-            const double2 u = reinterpret_cast<const double2*>(in.quad[lane])[0];
-            const double2 v = reinterpret_cast<const double2*>(in.quad[lane])[1];
-            quad[0] = u.x, quad[1] = u.y, quad[2] = v.x, quad[3] = v.y;
-          }
+          get_quad(in.quad[lane], quad[0], quad[1], quad[2], quad[3]);
           const uint32_t wrd = in.cw[lane];
           const T px = quad[0], py = quad[1], uz_in = in.uz[lane];
           const int elem = in.elem[lane];  // (tracked ids)
-          start_pass(a, ring + (slot ^ 2), lane, ring[slot ^ 2].elem[lane]);
-          start_elem<GATHER>(a, ring + slot, lane, take(ka));
+          PassBuf<T>* ahead = buf(at >= 2 * STRIDE ? at - 2 * STRIDE : at + 2 * STRIDE);
+          start_pass(a, ahead, lane, ahead->elem[lane]);
+          start_elem<GATHER>(a, buf(at), lane, take(ka));
           end_group();
-          slot = (slot + 1) & 3;
+          at = at == 3 * STRIDE ? 0u : at + STRIDE;
           const bool valid = p < end;
-          const bool sp = (int)wrd < 0;
+          const T* sp = sm.spc[valid ? (int)(wrd >> 31) : 2];
           // gather and Boris rotation (kernels_push.cuh: push_core, the same operations)
           T ex, ey, ez, bx, by, bz;
           if constexpr (F32) {
@@ -440,7 +495,9 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
             ex = coef_at(rc, px, py), ey = coef_at(rc + 4, px, py), ez = coef_at(rc + 8, px, py);
             bx = coef_at(rc + 12, px, py), by = coef_at(rc + 16, px, py), bz = coef_at(rc + 20, px, py);
           }
-          const T c0 = sp ? a.c0[1] : a.c0[0], c1 = sp ? a.c1[1] : a.c1[0];
+          T c0, c1, qv, me;
+          get_quad(sp, c0, c1, qv, me);
+          const T mi = sp[4];
           const T umx = A::mad(c1, ex, quad[2]), umy = A::mad(c1, ey, quad[3]), umz = A::mad(c1, ez, uz_in);
           const T g2m = A::mad(umz, umz, A::mad(umy, umy, A::mad(umx, umx, one)));
           const T c2 = A::mul(c0, rsqrt_normal(g2m));
@@ -453,8 +510,7 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
           const T upx = A::mad(u0y, sz, A::mad(-u0z, sy, umx));
           const T upy = A::mad(u0z, sx, A::mad(-u0x, sz, umy));
           const T upz = A::mad(u0x, sy, A::mad(-u0y, sx, umz));
-          const T ux = A::mad(c1, ex, upx), uz = A::mad(c1, ez, upz);
-          T uy = A::mad(c1, ey, upy);
+          const T ux = A::mad(c1, ex, upx), uz = A::mad(c1, ez, upz); T uy = A::mad(c1, ey, upy);
           const T g2 = A::mad(uz, uz, A::mad(uy, uy, A::mad(ux, ux, one)));
           const T rg = rsqrt_normal(g2), gama = A::mul(g2, rg), c3 = A::mul(a.dtcva, rg);
           T x1 = A::mad(A::mul(c3, ux), a.idx, px), y1 = A::mad(A::mul(c3, uy), a.idy, py);
@@ -465,15 +521,14 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
           if constexpr (F32) {  // kinetic energy: (gamma - 1) m = u^2 m / (gamma + 1)
             const float usq = A::mad(uz, uz, A::mad(uy, uy, A::mul(ux, ux)));
             const float ke = div_normal(usq, A::add(gama, 1.0f));
-            pke_e = A::mad(ke, valid && sp ? a.ms[1] : 0.0f, pke_e);
-            pke_i = A::mad(ke, valid && !sp ? a.ms[0] : 0.0f, pke_i);
+            pke_e = A::mad(ke, me, pke_e);
+            pke_i = A::mad(ke, mi, pke_i);
           } else {
             const T ke = A::sub(gama, one);
-            pke_e = A::mad(ke, valid && sp ? a.ms[1] : T(0), pke_e);
-            pke_i = A::mad(ke, valid && !sp ? a.ms[0] : T(0), pke_i);
+            pke_e = A::mad(ke, me, pke_e);
+            pke_i = A::mad(ke, mi, pke_i);
           }
           {  // deposit (pic2d.f90:1237-1295), cell-relative and for unit charges: the whole move of a particle that stays
-            const T qv = valid ? (sp ? T(-1) : one) : T(0);
             const T qs = cross ? T(0) : qv;
             // twice the midpoint, from the cell centre; the factors 1/2 and the constant parts of the weights
             // enter with the cell's sums (cell_terms)
@@ -505,31 +560,29 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
             acc[15] = A::mad(qv, py, acc[15]);
             acc[16] = A::mad(qx, py, acc[16]);
           }
-          uint32_t cw = wrd;
           const unsigned mc = __ballot_sync(FULL, cross);
-          if (cross) {
-            if (A::abs(x1) > T(1.5) || A::abs(y1) > T(1.5)) status |= PBPIC_STATUS_CELL_JUMP;
+          uint32_t cw = wrd;
+          if (cross) {  // LATE: stored as it is, its new cell comes with the queue
             const int e = nq + __popc(mc & lanemask_lt());
-            q[e] = px;
-            q[PC_QUEUE + e] = py;
-            q[2 * PC_QUEUE + e] = x1;
-            q[3 * PC_QUEUE + e] = y1;
-            qw[e] = wrd;
-            const int dcx = cell_step(x1), dcy = cell_step(y1);
-            x1 = A::sub(x1, (T)dcx);
-            y1 = A::sub(y1, (T)dcy);
-            cw = wrd + (uint32_t)(dcx * 65536 + dcy);
-            if (edge) {  // boundaries (kernels_push.cuh: push_core)
-              int nix = ixt + dcx, niy = y0 + row + dcy;
-              nix = nix < 0 ? nix + a.mx : (nix >= a.mx ? nix - a.mx : nix);
-              if (a.ybc == 0) {
-                niy = niy < 0 ? niy + a.my : (niy >= a.my ? niy - a.my : niy);
-              } else if (niy < 0 || niy >= a.my) {
-                niy = niy < 0 ? 0 : a.my - 1;
-                y1 = -y1;
-                uy = -uy;
+            set_quad(q[e], px, py, x1, y1);
+            qw[e] = make_int2((int)wrd, p);
+            if constexpr (!LATE) {
+              const int dcx = cell_step(x1), dcy = cell_step(y1);
+              x1 = A::sub(x1, (T)dcx);
+              y1 = A::sub(y1, (T)dcy);
+              cw = wrd + (uint32_t)(dcx * 65536 + dcy);
+              if (edge) {  // boundaries (kernels_push.cuh: push_core)
+                int nix = ixt + dcx, niy = y0 + row + dcy;
+                nix = nix < 0 ? nix + a.mx : (nix >= a.mx ? nix - a.mx : nix);
+                if (a.ybc == 0) {
+                  niy = niy < 0 ? niy + a.my : (niy >= a.my ? niy - a.my : niy);
+                } else if (niy < 0 || niy >= a.my) {
+                  niy = niy < 0 ? 0 : a.my - 1;
+                  y1 = -y1;
+                  uy = -uy;
+                }
+                cw = (wrd & 0x80000000u) | ((uint32_t)nix << 16) | (uint32_t)niy;
               }
-              cw = (wrd & 0x80000000u) | ((uint32_t)nix << 16) | (uint32_t)niy;
             }
           }
           if (valid) {
@@ -541,7 +594,7 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
           nq += __popc(mc);
           if (nq >= 32) {
             nq -= 32;
-            drain_crossers<T>(w, q, qw, nq, 32);
+            status |= drain_crossers<T, LATE>(w, q, qw, nq, 32);
           }
         } while (--chunk > 0);
         // the cell's sums so far to the window
@@ -570,7 +623,7 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
     } while (kc.left != 0x7fffffff);
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   }
-  if (nq) drain_crossers<T>(w, q, qw, 0, nq);
+  if (nq) status |= drain_crossers<T, LATE>(w, q, qw, 0, nq);
   if (F32 && !staged) mbar_wait(&sm.mbar, parity);  // not in flight when the shared memory is reused
 
   // fold the window into the global current; the tile's counts and energies

@@ -844,32 +844,19 @@ int do_store_grid(pbpic_handle* h, double* g8) {
 
 int do_store_denjr(pbpic_handle* h, double* j4) {
   const int64_t pe = plane_elems(h);
-  std::vector<double> acc((size_t)(4 * pe));
-  CK(cudaMemcpyAsync(acc.data(), h->jacc, (size_t)(4 * pe) * 8, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
   const pbpic_config& c = h->cfg;
-  double sc[4];
-  if (h->mixed) {
-    sc[0] = c.in0 * (c.dx / c.dt) * FIX_INV;
-    sc[1] = c.in0 * (c.dy / c.dt) * FIX_INV;
-    sc[2] = c.in0 * c.cva * FIX_INV;
-    sc[3] = c.in0 * FIX_INV;
-  } else {
-    for (int k = 0; k < 4; ++k) sc[k] = c.in0;
-  }
-  for (int comp = 0; comp < 4; ++comp)
-    for (int64_t k = 0; k < pe; ++k) {
-      const size_t i = (size_t)comp * pe + k;
-      double v;
-      if (h->mixed) {
-        long long q;
-        memcpy(&q, &acc[i], 8);
-        v = (double)q;
-      } else {
-        v = acc[i];
-      }
-      j4[i] = v * sc[comp];
-    }
+  double4 sc = make_double4(c.in0, c.in0, c.in0, c.in0);
+  if (h->mixed)
+    sc = make_double4(c.in0 * (c.dx / c.dt) * FIX_INV, c.in0 * (c.dy / c.dt) * FIX_INV, c.in0 * c.cva * FIX_INV,
+                      c.in0 * FIX_INV);
+  // The scaled current lies in the next push's accumulators, which that push then clears itself.
+  h->j2_clear = false;
+  double* out = (double*)h->jacc2;
+  if (h->mixed) k_denjr<long long><<<grid_for(4 * pe, 256), 256, 0, h->stream>>>(pe, (const long long*)h->jacc, sc, out);
+  else k_denjr<double><<<grid_for(4 * pe, 256), 256, 0, h->stream>>>(pe, (const double*)h->jacc, sc, out);
+  CKLAUNCH("k_denjr");
+  CK(cudaMemcpyAsync(j4, out, (size_t)(4 * pe) * 8, cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
   return PBPIC_OK;
 }
 
