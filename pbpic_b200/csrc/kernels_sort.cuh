@@ -349,6 +349,7 @@ struct FusedSortParams {
   int32_t* counts;         // [mx*my + 1] per-cell counts (last entry 0)
   int32_t* off;            // exclusive scan of counts
   int32_t* base;           // [ntiles][nb] first slot of each (tile, bin)
+  int32_t* sums;           // batched: the chunks' totals, then their exclusive scan
 };
 
 // The (tile, bin) entries of a cell: the tiles whose windows hold it are those of
@@ -422,24 +423,34 @@ __device__ __forceinline__ void fused_slots(const FusedSortParams& a, int c, int
   }
 }
 
-// The fused sort's tables in two launches. k_counts_scan: the cell counts of a chunk of
-// CS_TILE cells and their exclusive scan within it, and the chunk's total.
-// k_fused_offsets: every block sums the totals before its chunk itself (they are
-// a few KB in L2), completes the chunk's offsets and gives each (tile, bin) its
-// first slot (the offset plus the cell's particles in earlier tiles) and each tile its position range. `scanned`: the totals are
-// already prefix sums (more than CS_MAXCHUNKS chunks).
+// The fused sort's tables. Chunks of CS_TILE cells: the cell counts and their exclusive scan
+// within the chunk (chunk_counts), then, with the particles before the chunk known, the cells'
+// offsets, each (tile, bin)'s first slot (the offset plus the cell's particles in
+// earlier tiles) and each tile's position range (chunk_tables).
 //
-// Latency-bound, 5-6 us each on 64x64 cells; counts, chunk scan, scan of the totals, offsets
-// and tile ranges were five launches of together 41 us there. Chunks of 1024 cells
-// so that 131 thousand cells still fill 128 blocks.
+// Up to CS_MAXCHUNKS chunks one launch does both (k_fused_tables): every block leaves its chunk's
+// total with a mark in `words` and adds up those before its own, which are a few KB in L2.
+// A block that has waited long enough counts the missing chunk's cells itself, so no
+// order of the blocks is assumed.
+// Latency-bound: two launches took 4.5 + 6.4 us and the gap between them on 128x128 cells, one
+// 8.9 us; the step 57.0 -> 55.1 us there, 36.8 -> 33.4 us on 64x64 cells, 74.3 -> 71.3 us on
+// 193x131. Beyond, k_counts_scan and k_fused_offsets
+// with the totals scanned between them: there a block's sum over all the totals before it would grow with the
+// square of the chunks. Chunks of 1024 cells so that 131 thousand cells still fill 128 blocks.
 constexpr int CS_BT = 256, CS_IPT = 4, CS_TILE = CS_BT * CS_IPT;
 constexpr int CS_MAXCHUNKS = 8192;
+constexpr int CS_POLLS = 1 << 16;
 
-static __global__ void __launch_bounds__(CS_BT) k_counts_scan(FusedSortParams a, int32_t* sums) {
-  __shared__ int32_t buf[CS_TILE];
-  __shared__ int32_t ws[CS_BT / 32];
+struct ChunkSmem {
+  int32_t buf[CS_TILE];  // the chunk's counts, then their scan
+  int32_t ws[CS_BT / 32];
+};
+
+// Counts and their scan within the chunk (in sm.buf); the chunk's total, in the last thread.
+__device__ __forceinline__ int32_t chunk_counts(const FusedSortParams& a, int64_t chunk, ChunkSmem& sm) {
+  int32_t(&buf)[CS_TILE] = sm.buf;
   const int t = threadIdx.x;
-  const int64_t ncells = (int64_t)a.mx * a.my, base = (int64_t)blockIdx.x * CS_TILE;
+  const int64_t ncells = (int64_t)a.mx * a.my, base = chunk * CS_TILE;
 #pragma unroll
   for (int k = 0; k < CS_IPT; ++k) {
     const int64_t c = base + k * CS_BT + t;
@@ -460,63 +471,113 @@ static __global__ void __launch_bounds__(CS_BT) k_counts_scan(FusedSortParams a,
     const int32_t y = __shfl_up_sync(FULL, inc, d);
     if ((int)lane_id() >= d) inc += y;
   }
-  if (lane_id() == 31) ws[t >> 5] = inc;
+  if (lane_id() == 31) sm.ws[t >> 5] = inc;
   __syncthreads();
   int32_t before = 0;
 #pragma unroll
-  for (int k = 0; k < CS_BT / 32; ++k) before += k < (t >> 5) ? ws[k] : 0;
+  for (int k = 0; k < CS_BT / 32; ++k) before += k < (t >> 5) ? sm.ws[k] : 0;
   const int32_t excl = before + inc - s;
 #pragma unroll
   for (int k = 0; k < CS_IPT; ++k) buf[t * CS_IPT + k] = excl + v[k];
   __syncthreads();
-#pragma unroll
-  for (int k = 0; k < CS_IPT; ++k) {
-    const int64_t c = base + k * CS_BT + t;
-    if (c <= ncells) a.off[c] = buf[k * CS_BT + t];
-  }
-  if (t == CS_BT - 1) sums[blockIdx.x] = before + inc;
+  return before + inc;
 }
 
-static __global__ void __launch_bounds__(CS_BT) k_fused_offsets(FusedSortParams a, const int32_t* sums, bool scanned,
-                                                                int32_t* tile_off) {
-  __shared__ int32_t ws[CS_BT / 32];
-  const int t = threadIdx.x;
-  const int64_t ncells = (int64_t)a.mx * a.my, base = (int64_t)blockIdx.x * CS_TILE;
-  int32_t prefix = 0;
-  if (scanned) {
-    prefix = sums[blockIdx.x];
-  } else {
-    for (int k = t; k < (int)blockIdx.x; k += CS_BT) prefix += sums[k];
-    prefix = __reduce_add_sync(FULL, prefix);
-    if (lane_id() == 0) ws[t >> 5] = prefix;
-    __syncthreads();
-    prefix = 0;
-#pragma unroll
-    for (int k = 0; k < CS_BT / 32; ++k) prefix += ws[k];
+// The tables of cell c, whose particles start at `o` (c = ncells: the end).
+__device__ __forceinline__ void chunk_tables(const FusedSortParams& a, int64_t c, int32_t o, int32_t* tile_off) {
+  a.off[c] = o;
+  if (c == (int64_t)a.mx * a.my) {
+    tile_off[a.ntiles] = o;
+    return;
   }
-#pragma unroll
-  for (int k = 0; k < CS_IPT; ++k) {
-    const int64_t c = base + k * CS_BT + t;
-    if (c > ncells) continue;
-    const int32_t o = a.off[c] + prefix;
-    a.off[c] = o;
-    if (c == ncells) {
-      tile_off[a.ntiles] = o;
-      continue;
+  const int cx = (int)c / a.my, cy = (int)c - cx * a.my;
+  if (cy % a.ty == 0) tile_off[cx * a.tpc + cy / a.ty] = o;
+  fused_slots(a, (int)c, o);
+}
+
+// words: [0] blocks done, then a word per chunk (its total, marked in bit 32);
+// all zero before, and after.
+static __global__ void __launch_bounds__(CS_BT) k_fused_tables(FusedSortParams a, unsigned long long* words,
+                                                               int32_t* tile_off) {
+  __shared__ ChunkSmem sm;
+  __shared__ int32_t part[CS_BT / 32];
+  __shared__ int done;
+  const int t = threadIdx.x, chunk = blockIdx.x;
+  volatile unsigned long long* totals = words + 1;
+  const int32_t total = chunk_counts(a, chunk, sm);
+  if (t == CS_BT - 1) totals[chunk] = (1ull << 32) | (unsigned)total;
+  const int64_t ncells = (int64_t)a.mx * a.my, base = (int64_t)chunk * CS_TILE;
+  int32_t before = 0;
+  for (int k = t; k < chunk; k += CS_BT) {
+    unsigned long long v = totals[k];
+    for (int polls = 0; !(v >> 32) && polls < CS_POLLS; ++polls) v = totals[k];
+    if (v >> 32) {
+      before += (int32_t)v;
+    } else {
+      const int64_t c0 = (int64_t)k * CS_TILE, c1 = min(c0 + CS_TILE, ncells);
+      for (int64_t c = c0; c < c1; ++c) before += fused_count(a, (int)c);
     }
-    const int cx = (int)c / a.my, cy = (int)c - cx * a.my;
-    if (cy % a.ty == 0) tile_off[cx * a.tpc + cy / a.ty] = o;
-    fused_slots(a, (int)c, o);
+  }
+  before = __reduce_add_sync(FULL, before);
+  if (lane_id() == 0) part[t >> 5] = before;
+  __syncthreads();
+  before = 0;
+#pragma unroll
+  for (int k = 0; k < CS_BT / 32; ++k) before += part[k];
+#pragma unroll
+  for (int k = 0; k < CS_IPT; ++k) {
+    const int64_t c = base + k * CS_BT + t;
+    if (c <= ncells) chunk_tables(a, c, before + sm.buf[k * CS_BT + t], tile_off);
+  }
+  // every block has read the totals once all are done: the last one clears them
+  if (t == 0) done = (int)atomicAdd(&words[0], 1ull);
+  __syncthreads();
+  if (done != (int)gridDim.x - 1) return;
+  for (int k = t; k < (int)gridDim.x + 1; k += CS_BT) words[k] = 0ull;
+}
+
+static __global__ void __launch_bounds__(CS_BT) k_counts_scan(FusedSortParams a, int32_t* sums) {
+  __shared__ ChunkSmem sm;
+  const int64_t ncells = (int64_t)a.mx * a.my, base = (int64_t)blockIdx.x * CS_TILE;
+  const int32_t total = chunk_counts(a, blockIdx.x, sm);
+#pragma unroll
+  for (int k = 0; k < CS_IPT; ++k) {
+    const int64_t c = base + k * CS_BT + threadIdx.x;
+    if (c <= ncells) a.off[c] = sm.buf[k * CS_BT + threadIdx.x];
+  }
+  if (threadIdx.x == CS_BT - 1) sums[blockIdx.x] = total;
+}
+
+// `sums`: prefix sums of the chunks' totals.
+static __global__ void __launch_bounds__(CS_BT) k_fused_offsets(FusedSortParams a, const int32_t* sums,
+                                                                int32_t* tile_off) {
+  const int64_t ncells = (int64_t)a.mx * a.my, base = (int64_t)blockIdx.x * CS_TILE;
+  const int32_t prefix = sums[blockIdx.x];
+#pragma unroll
+  for (int k = 0; k < CS_IPT; ++k) {
+    const int64_t c = base + k * CS_BT + threadIdx.x;
+    if (c <= ncells) chunk_tables(a, c, a.off[c] + prefix, tile_off);
   }
 }
 
-static __global__ void k_fused_counts_batched(const FusedSortParams* d) {
+// Batched domains: the tables in three launches (grid row blockIdx.y = domain), the chunks'
+// totals scanned between (k_scan_batched).
+static __global__ void __launch_bounds__(CS_BT) k_fused_counts_batched(const FusedSortParams* d) {
   __shared__ FusedSortParams a;
+  __shared__ ChunkSmem sm;
   if (threadIdx.x == 0) a = d[blockIdx.y];
   __syncthreads();
-  const int ncells = a.mx * a.my;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncells; c += gridDim.x * blockDim.x)
-    a.counts[c] = c == ncells ? 0 : fused_count(a, c);
+  const int64_t ncells = (int64_t)a.mx * a.my;
+  for (int64_t chunk = blockIdx.x; chunk * CS_TILE <= ncells; chunk += gridDim.x) {
+    const int32_t total = chunk_counts(a, chunk, sm);
+    if (threadIdx.x == CS_BT - 1) a.sums[chunk] = total;
+#pragma unroll
+    for (int k = 0; k < CS_IPT; ++k) {
+      const int64_t c = chunk * CS_TILE + k * CS_BT + threadIdx.x;
+      if (c <= ncells) a.off[c] = sm.buf[k * CS_BT + threadIdx.x];
+    }
+    __syncthreads();
+  }
 }
 
 static __global__ void k_fused_base_batched(const FusedSortParams* d) {
@@ -524,7 +585,11 @@ static __global__ void k_fused_base_batched(const FusedSortParams* d) {
   if (threadIdx.x == 0) a = d[blockIdx.y];
   __syncthreads();
   const int ncells = a.mx * a.my;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += gridDim.x * blockDim.x) fused_slots(a, c, a.off[c]);
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c <= ncells; c += gridDim.x * blockDim.x) {
+    const int32_t o = a.off[c] + a.sums[c / CS_TILE];
+    a.off[c] = o;
+    if (c < ncells) fused_slots(a, c, o);
+  }
 }
 
 template <class T>
@@ -538,12 +603,6 @@ struct ScatterParams {
 
 constexpr int SC_MAXNB = 3 * (64 + 2) + 1;  // window bins of the largest tile, plus a sentinel
 
-// Per-warp bin counts and the block's running ranks of one tile.
-struct ScatterSmem {
-  int32_t cnt[8][SC_MAXNB];
-  int32_t run[SC_MAXNB], sbase[SC_MAXNB];
-};
-
 // ------------------------------------------------- permutation-only sort
 // The stable ranking of a tile's particles by new cell (warp match_any +
 // per-warp counters, array order), from the cell words only: the
@@ -551,14 +610,22 @@ struct ScatterSmem {
 // perm[d] = p. The particle data stay where they are; the next push reads
 // them through perm (PushParams::src), and a gather (k_gather) applies perm
 // when the arrays themselves must be in cell order.
+// Chunks of 256 threads x 8 particles: 26.2 M particles 70 us; 256 x 16 75, 256 x 12 76, 512 x 8 75,
+// 512 x 4 92, 128 x 16 79 (blocks of 512 would save 1 us of 9 at 1 M).
 #ifndef PBPIC_PERM_IPT
 #define PBPIC_PERM_IPT 8  // particles per thread in one chunk of the ranking
 #endif
-constexpr int SP_IPT = PBPIC_PERM_IPT, SP_CHUNK = 256 * SP_IPT;
+constexpr int SP_IPT = PBPIC_PERM_IPT, SP_BT = 256, SP_WARPS = SP_BT / 32, SP_CHUNK = SP_BT * SP_IPT;
+
+// Per-warp bin counts and the block's running ranks of one tile.
+struct ScatterSmem {
+  int32_t cnt[SP_WARPS][SC_MAXNB];
+  int32_t run[SC_MAXNB], sbase[SC_MAXNB];
+};
 
 template <class T>
 __device__ __forceinline__ void perm_tile(const ScatterParams<T>& a, const int t, ScatterSmem& sm) {
-  int32_t(&cnt)[8][SC_MAXNB] = sm.cnt;
+  int32_t(&cnt)[SP_WARPS][SC_MAXNB] = sm.cnt;
   int32_t* perm = a.perm;
   const int ixt = t / a.tpc, y0 = (t - ixt * a.tpc) * a.ty, y1 = min(y0 + a.ty, a.my);
   const int pbeg = a.tile_off[t], pend = a.tile_off[t + 1];
@@ -572,7 +639,7 @@ __device__ __forceinline__ void perm_tile(const ScatterParams<T>& a, const int t
     sm.sbase[b] = a.base[(int64_t)t * a.nb + b];
   }
   for (int c0 = pbeg; c0 < pend; c0 += SP_CHUNK) {
-    for (int e = threadIdx.x; e < 8 * SC_MAXNB; e += blockDim.x) (&cnt[0][0])[e] = 0;
+    for (int e = threadIdx.x; e < SP_WARPS * SC_MAXNB; e += blockDim.x) (&cnt[0][0])[e] = 0;
     __syncthreads();
     int bin[SP_IPT], pos[SP_IPT];
     uint32_t vc[SP_IPT];
@@ -616,7 +683,7 @@ __device__ __forceinline__ void perm_tile(const ScatterParams<T>& a, const int t
     for (int b = threadIdx.x; b < a.nb; b += blockDim.x) {
       int32_t r = sm.run[b];
 #pragma unroll
-      for (int ww = 0; ww < 8; ++ww) {
+      for (int ww = 0; ww < SP_WARPS; ++ww) {
         const int32_t c = cnt[ww][b];
         cnt[ww][b] = r;
         r += c;
@@ -636,7 +703,7 @@ __device__ __forceinline__ void perm_tile(const ScatterParams<T>& a, const int t
 }
 
 template <class T>
-__global__ void __launch_bounds__(256) k_fused_perm(ScatterParams<T> a) {
+__global__ void __launch_bounds__(SP_BT) k_fused_perm(ScatterParams<T> a) {
   __shared__ ScatterSmem sm;
   perm_tile(a, blockIdx.x, sm);
 }
@@ -649,7 +716,7 @@ static __global__ void k_iota(int32_t* perm, int64_t n) {
 
 // Batched permutation-only sort: persistent blocks over the (domain, tile) table.
 template <class T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(SP_BT)
     k_fused_perm_batched(const ScatterParams<T>* descs, const int2* tiles, int ntiles, int* counter) {
   __shared__ ScatterSmem sm;
   __shared__ ScatterParams<T> a;

@@ -209,6 +209,7 @@ struct pbpic_handle {
   bool j2_clear = false;
   int32_t *counts = nullptr, *off = nullptr, *tile_off = nullptr;
   int32_t* tile_off2 = nullptr;  // written by the fused sort while its ranking reads tile_off (then swapped)
+  unsigned long long* chunk_words = nullptr;  // k_fused_tables' chunk totals, zero between launches
   int* ticket = nullptr;         // k_field_step's count of finished blocks
   double *ke_part = nullptr, *fe_part = nullptr;
   int nfe = 0, nke = 0;
@@ -683,12 +684,16 @@ int do_fused_sort(pbpic_handle* h) {
   // cell counts and their chunk scan; then the offsets, the (tile, bin) first
   // slots and the new tile ranges (the ranking still reads the push's)
   const int64_t nchunks = ((int64_t)h->ncells + 1 + CS_TILE - 1) / CS_TILE;
-  k_counts_scan<<<(unsigned)nchunks, CS_BT, 0, s>>>(f, h->scan_scratch);
-  CKLAUNCH("k_counts_scan");
-  const bool scanned = nchunks > CS_MAXCHUNKS;
-  if (scanned) TRY(scan_excl(s, h->scan_scratch, nchunks, h->scan_scratch + nchunks + 1));
-  k_fused_offsets<<<(unsigned)nchunks, CS_BT, 0, s>>>(f, h->scan_scratch, scanned, h->tile_off2);
-  CKLAUNCH("k_fused_offsets");
+  if (nchunks <= CS_MAXCHUNKS) {
+    k_fused_tables<<<(unsigned)nchunks, CS_BT, 0, s>>>(f, h->chunk_words, h->tile_off2);
+    CKLAUNCH("k_fused_tables");
+  } else {
+    k_counts_scan<<<(unsigned)nchunks, CS_BT, 0, s>>>(f, h->scan_scratch);
+    CKLAUNCH("k_counts_scan");
+    TRY(scan_excl(s, h->scan_scratch, nchunks, h->scan_scratch + nchunks + 1));
+    k_fused_offsets<<<(unsigned)nchunks, CS_BT, 0, s>>>(f, h->scan_scratch, h->tile_off2);
+    CKLAUNCH("k_fused_offsets");
+  }
   ScatterParams<T> sp{};  // the ranking reads the cell words and the tables only
   sp.mx = f.mx;
   sp.my = f.my;
@@ -702,7 +707,7 @@ int do_fused_sort(pbpic_handle* h) {
   if (n > 0) {  // the sorted order as a permutation; the particle data stay in place
     if (!h->perm) TRY(dalloc(h, &h->perm, ((size_t)std::max<int64_t>(h->cap, 1) + 16) * 4));
     sp.perm = h->perm;
-    k_fused_perm<T><<<h->ntiles, 256, 0, s>>>(sp);
+    k_fused_perm<T><<<h->ntiles, SP_BT, 0, s>>>(sp);
     CKLAUNCH("k_fused_perm");
     h->lazy = true;
   }
@@ -1125,11 +1130,12 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
   A(&h->fe_part, (size_t)std::max(h->nfe, field_tiles(c.mx, c.my)) * 2 * 8);
   A(&h->status, 16);
   A(&h->rhist, (size_t)radix_hist_ints((int64_t)capn) * 4);
-  // (the fused sort's chunk totals and, beyond CS_MAXCHUNKS of them, the levels of their scan)
+  // (beyond CS_MAXCHUNKS chunks, the fused sort's chunk totals and the levels of their scan)
   const int64_t nchunks = ((int64_t)h->ncells + 1 + CS_TILE - 1) / CS_TILE;
   const int64_t sc = std::max({scan_scratch_ints(radix_hist_ints((int64_t)capn)), scan_scratch_ints(h->ncells + 1),
                                nchunks + 1 + scan_scratch_ints(nchunks)});
   A(&h->scan_scratch, (size_t)sc * 4);
+  A(&h->chunk_words, (size_t)(CS_MAXCHUNKS + 1) * 8);
   A(&h->rho, (size_t)pe * 8);
   A(&h->dscalar, 64);  // scalars of the diagnostics (up to 4 doubles)
   if (r != PBPIC_OK) {
@@ -1144,6 +1150,7 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
   cudaMemset(h->off, 0, (size_t)(h->ncells + 1) * 4);
   cudaMemset(h->status, 0, 16);
   cudaMemset(h->ticket, 0, 16);
+  cudaMemset(h->chunk_words, 0, (size_t)(CS_MAXCHUNKS + 1) * 8);
   if (ensure_hist(h, 64) != PBPIC_OK || set_unsorted_tiles(h) != PBPIC_OK) {
     pbpic_destroy(h);
     return PBPIC_ENOMEM;
@@ -1637,7 +1644,7 @@ struct pbpic_batch {
   int ncells_tiles = 0, cells_blocks = 0;  // the table's first tiles: those pushed cell by cell
   bool track = false;                      // some domain carries particle ids
   size_t push_smem = 0, cells_smem = 0;
-  int gx_zero = 1, gx_cells = 1, gx_tiles = 1, gx_field = 1, gx_nodes = 1;
+  int gx_zero = 1, gx_cells = 1, gx_chunks = 1, gx_tiles = 1, gx_field = 1, gx_nodes = 1;
 };
 
 namespace {
@@ -1776,10 +1783,11 @@ int batch_layout(pbpic_batch* b) {
                                                : (const void*)k_push_batched<float, true, true, 2, false, true>);
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, PushThreads<float>::value, smem));
   b->push_blocks = std::max(1, std::min(b->ntiles - b->ncells_tiles, sms * std::max(1, per_sm)));
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused_perm_batched<float>, 256, 0));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused_perm_batched<float>, SP_BT, 0));
   b->scatter_blocks = std::max(1, std::min(b->ntiles, sms * std::max(1, per_sm)));
   b->gx_zero = grid_for(maxacc, 256, 1024);
   b->gx_cells = grid_for(maxcells, 256);
+  b->gx_chunks = grid_for(maxcells + 1, CS_TILE);
   b->gx_tiles = grid_for(maxtiles, 256, 1 << 16);
   b->gx_field = grid_for(maxfield, 256);
   b->gx_nodes = maxnodes;
@@ -1834,6 +1842,7 @@ int batch_descriptors(pbpic_batch* b) {
     f.ntiles = h->ntiles;
     f.nb = h->nb;
     f.tilecnt = h->tilecnt;
+    f.sums = h->scan_scratch;
     f.counts = h->counts;
     f.off = h->off;
     f.base = h->tbase;
@@ -1849,9 +1858,8 @@ int batch_descriptors(pbpic_batch* b) {
     BatchDomain& bd = b->h_dom[d];
     bd.jacc = (long long*)h->jacc;
     bd.nacc = 4 * plane_elems(h);
-    bd.counts = h->counts;
-    bd.off = h->off;
-    bd.ncounts = h->ncells + 1;
+    bd.sums = h->scan_scratch;
+    bd.nsums = (int)(((int64_t)h->ncells + 1 + CS_TILE - 1) / CS_TILE);
     EnergyRow& e = b->h_erow[d];
     e.ke_part = h->ke_part;
     e.nke = h->ntiles;
@@ -1893,13 +1901,13 @@ int batch_enqueue_step(pbpic_batch* b, int par) {
     else b->compat ? run(k_push_batched<float, true, true, 2, true, true>) : run(k_push_batched<float, true, true, 2, false, true>);
     CKLAUNCH("k_push_batched");
   }
-  k_fused_counts_batched<<<dim3(b->gx_cells, D), 256, 0, s>>>(b->d_fsort);
+  k_fused_counts_batched<<<dim3(b->gx_chunks, D), CS_BT, 0, s>>>(b->d_fsort);
   CKLAUNCH("k_fused_counts_batched");
   k_scan_batched<<<D, SCB, 0, s>>>(b->d_dom);
   CKLAUNCH("k_scan_batched");
   k_fused_base_batched<<<dim3(b->gx_cells, D), 256, 0, s>>>(b->d_fsort);
   CKLAUNCH("k_fused_base_batched");
-  k_fused_perm_batched<float><<<b->scatter_blocks, 256, 0, s>>>(b->d_scat + (size_t)par * D, b->d_tiles,
+  k_fused_perm_batched<float><<<b->scatter_blocks, SP_BT, 0, s>>>(b->d_scat + (size_t)par * D, b->d_tiles,
                                                                 b->ntiles, ctr + 1);
   CKLAUNCH("k_fused_perm_batched");
   k_tile_off_batched<<<dim3(b->gx_tiles, D), 256, 0, s>>>(b->d_toff);

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import pbpic_b200
+from pbpic_b200 import configs
 from test_gpu_edges import rows_of
 from test_gpu_parity import field_err, new_sim, plasma, random_fields
 
@@ -67,5 +68,32 @@ def test_sort_tables(gpu_lib, oracle_mod, ybc, mx, my, ty):
             post = s.particles()
             order = np.argsort(pre["grid"], kind="stable")
             assert np.array_equal(post["pid"], pre["pid"][order])
+            assert np.array_equal(s.cell_counts(), np.bincount(pre["grid"] - 1, minlength=mx * my))
+        assert s.status() == 0
+
+
+@pytest.mark.parametrize("mx,my", [(31, 33), (32, 32), (25, 41), (64, 80), (4096, 2049)])
+def test_sort_tables_chunks(gpu_lib, mx, my):
+    """Cells one less than, equal to and one more than a chunk of the tables, several chunks, and more
+    than one launch takes: the order and counts exactly, twice (the chunks' totals are cleared)."""
+    rng = np.random.default_rng(mx * my)
+    n = 20000
+    p = np.zeros(n, dtype=pbpic_b200._lib.PARTICLE_F64)
+    p["grid"] = rng.integers(0, mx * my, n) + 1
+    p["q"] = np.where(np.arange(n) % 2, 1, -1)
+    p["pid"] = np.arange(n)
+    for c, w in (("dx", 0.49), ("dy", 0.49), ("ux", 0.8), ("uy", 0.8), ("uz", 0.8)):
+        p[c] = rng.uniform(-w, w, n)
+    cfg, _ = configs.uniform_c1(mx=mx, my=my)
+    with new_sim(cfg, n, precision="fp32", options=pbpic_b200.OPT_NO_AUTOSORT) as s:
+        s.load_particles(p)
+        s.countingsort()
+        for _ in range(2):
+            s.pusher()
+            pre = s.particles()
+            s.countingsort()
+            post = s.particles()
+            assert (np.diff(pre["grid"]) < 0).any()
+            assert np.array_equal(post["pid"], pre["pid"][np.argsort(pre["grid"], kind="stable")])
             assert np.array_equal(s.cell_counts(), np.bincount(pre["grid"] - 1, minlength=mx * my))
         assert s.status() == 0
