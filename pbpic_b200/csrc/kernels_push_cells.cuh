@@ -298,19 +298,28 @@ __device__ __forceinline__ void group_sums(T (&v)[16]) {
 }
 
 // Bilinear coefficients (A, B, C, D) of the 6 fields over a cell, from the node grid
-// (kernels_field.cuh: cell_record).
+// (kernels_field.cuh: cell_record). A is the correctly rounded mean (its sums' rounding errors are carried), and
+// coef_at adds it last, so that the gather is no further off than the sum of four
+// weighted nodes: rms error 6.9e-17 of the field against 7.4e-17 for nodes that differ by a tenth,
+// 7.8e-17 against 7.9e-17 for uncorrelated Yee values averaged to nodes (9.9e-17 with a plain
+// mean added first).
 __device__ __forceinline__ void cell_coefs(const PushParams<double>& a, int ix, int iy, int f, double* r) {
   const double* g = a.ng + ((long long)ix * (a.my + 1) + iy) * 8 + (f < 3 ? f : f + 1);
   const double* h = g + (long long)(a.my + 1) * 8;
   const double n00 = __ldg(g), n01 = __ldg(g + 8), n10 = __ldg(h), n11 = __ldg(h + 8);
-  r[0] = 0.25 * ((n00 + n01) + (n10 + n11));
-  r[1] = 0.5 * ((n10 + n11) - (n00 + n01));
-  r[2] = 0.5 * ((n01 + n11) - (n00 + n10));
+  auto err = [](double a, double b, double s) {  // a + b - s, s = a + b rounded (Knuth's two-sum)
+    const double t = s - a;
+    return (a - (s - t)) + (b - t);
+  };
+  const double s0 = n00 + n01, s1 = n10 + n11, s = s0 + s1;
+  r[0] = 0.25 * (s + (err(s0, s1, s) + (err(n00, n01, s0) + err(n10, n11, s1))));
+  r[1] = 0.5 * ((n10 - n00) + (n11 - n01));
+  r[2] = 0.5 * ((n01 - n00) + (n11 - n10));
   r[3] = (n11 - n10) - (n01 - n00);
 }
 __device__ __forceinline__ double coef_at(const double* r, double x, double y) {
   const double2 ab = reinterpret_cast<const double2*>(r)[0], cd = reinterpret_cast<const double2*>(r)[1];
-  return __fma_rn(__fma_rn(cd.y, x, cd.x), y, __fma_rn(ab.y, x, ab.x));
+  return __dadd_rn(__fma_rn(__fma_rn(cd.y, x, cd.x), y, __dmul_rn(ab.y, x)), ab.x);
 }
 
 // Push of tile t by all threads of the block (kernels_push.cuh: push_tile).
