@@ -1211,6 +1211,7 @@ __global__ void __launch_bounds__(PushThreads<T>::value, MIXED ? PBPIC_PUSH_MINB
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ PushSmem<T, MIXED> sm;
   if (threadIdx.x == 0) mbar_init(&sm.mbar);  // thread 0 also starts the copy; the others wait after a barrier
+  cudaTriggerProgrammaticLaunchCompletion();  // (pbpic_api.cu: launch_early)
   push_tile<T, MIXED, HIST, MIXED ? PBPIC_PUSH_HALVES : PBPIC_PUSH_HALVES_FP64, COMPAT, GATHER>(a, blockIdx.x, sm,
                                                                                               smem_raw, 0u);
 }

@@ -675,6 +675,7 @@ __global__ void __launch_bounds__(PC_THREADS, cells_minblocks(sizeof(T) == 4)) k
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ CellsSmem<T> sm;
   if (sizeof(T) == 4 && threadIdx.x == 0) mbar_init(&sm.mbar);
+  cudaTriggerProgrammaticLaunchCompletion();  // (pbpic_api.cu: launch_early)
   push_cells<T, L, GATHER, PID>(a, blockIdx.x, sm, smem_raw, 0u);
 }
 

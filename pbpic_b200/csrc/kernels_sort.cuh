@@ -502,6 +502,7 @@ static __global__ void __launch_bounds__(CS_BT) k_fused_tables(FusedSortParams a
   __shared__ ChunkSmem sm;
   __shared__ int32_t part[CS_BT / 32];
   __shared__ int done;
+  cudaGridDependencySynchronize();
   const int t = threadIdx.x, chunk = blockIdx.x;
   volatile unsigned long long* totals = words + 1;
   const int32_t total = chunk_counts(a, chunk, sm);
@@ -529,6 +530,8 @@ static __global__ void __launch_bounds__(CS_BT) k_fused_tables(FusedSortParams a
     const int64_t c = base + k * CS_BT + t;
     if (c <= ncells) chunk_tables(a, c, before + sm.buf[k * CS_BT + t], tile_off);
   }
+  // (not earlier: the ranking's waiting blocks would take the field solve's places, 68 -> 78 us a step of sparse beams)
+  cudaTriggerProgrammaticLaunchCompletion();
   // every block has read the totals once all are done: the last one clears them
   if (t == 0) done = (int)atomicAdd(&words[0], 1ull);
   __syncthreads();
@@ -705,6 +708,7 @@ __device__ __forceinline__ void perm_tile(const ScatterParams<T>& a, const int t
 template <class T>
 __global__ void __launch_bounds__(SP_BT) k_fused_perm(ScatterParams<T> a) {
   __shared__ ScatterSmem sm;
+  cudaGridDependencySynchronize();
   perm_tile(a, blockIdx.x, sm);
 }
 

@@ -53,6 +53,24 @@ int fail(int code, const std::string& msg) {
     if (e_ != cudaSuccess) return fail(PBPIC_ECUDA, std::string(what) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// A launch whose blocks may take their places while the kernel before it in the stream is finishing (once all of
+// that one's blocks have started or, the sort's tables, are done); the kernel waits for its results itself
+// (cudaGridDependencySynchronize), so the start-up of the sort's two launches lies under the push and the tables. Step: 64x64
+// cells 33.4 -> 32.5 us, 128x128 55.0 -> 51.2 us, FP64 76.8 -> 74.0 us, 193x131 71.2 -> 68.0 us, 512x256 442 -> 438 us.
+template <class... P, class... A>
+void launch_early(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);  // (an error is found by CKLAUNCH)
+}
+
 #define TRY(...)                   \
   do {                             \
     int r_ = (__VA_ARGS__);        \
@@ -358,11 +376,11 @@ Comps<T> C(pbpic_handle* h, int buf) {
 // Lanes per cell of the push cell by cell (kernels_push_cells.cuh: sorted input, no compat
 // switch, not the exact order), 0 for the tile push. By the domain's mean particles
 // per cell, uniform plasma on 512x256 cells, us per step.
-// Mixed, tile push / 16 lanes / 32 lanes: 8: 168 / 178 / 206; 16: 186 / 189 / 220;
-// 24: 207 / 192 / 220; 64: 307 / 253 / 284; 128: 484 / 343 / 363; 200: 664 / 468 / 472
-// (a Harris sheet of 200: 16 lanes 518, 32 lanes 505).
-// Plain, tile push / 32 lanes (16 lanes never better): 16: 244 / 293; 24: 286 / 304;
-// 64: 501 / 399; 128: 826 / 556; 180: 1097 / 685.
+// Mixed, tile push / 16 lanes / 32 lanes: 8: 123 / 133 / 169; 12: 118 / 130 / 172;
+// 16: 133 / 136 / 168; 20: 153 / 136 / 168; 64: 269 / 197 / 230; 128: 446 / 309 / 320;
+// 200: 625 / 443 / 429 (a Harris sheet of 200: 670 / 458 / 439).
+// Plain, tile push / 32 lanes (16 lanes never better): 16: 187 / 234; 24: 231 / 251;
+// 32: 269 / 272; 64: 429 / 345; 128: 748 / 494; 180: 1007 / 625.
 int cells_lanes(const pbpic_handle* h) {
   if (h->cfg.compat != 0 || (!h->mixed && (h->cfg.options & PBPIC_OPT_EXACT_FP64))) return 0;
   const double per_cell = (double)h->n / (double)h->ncells;
@@ -685,7 +703,7 @@ int do_fused_sort(pbpic_handle* h) {
   // slots and the new tile ranges (the ranking still reads the push's)
   const int64_t nchunks = ((int64_t)h->ncells + 1 + CS_TILE - 1) / CS_TILE;
   if (nchunks <= CS_MAXCHUNKS) {
-    k_fused_tables<<<(unsigned)nchunks, CS_BT, 0, s>>>(f, h->chunk_words, h->tile_off2);
+    launch_early(k_fused_tables, (unsigned)nchunks, CS_BT, s, f, h->chunk_words, h->tile_off2);
     CKLAUNCH("k_fused_tables");
   } else {
     k_counts_scan<<<(unsigned)nchunks, CS_BT, 0, s>>>(f, h->scan_scratch);
@@ -707,7 +725,7 @@ int do_fused_sort(pbpic_handle* h) {
   if (n > 0) {  // the sorted order as a permutation; the particle data stay in place
     if (!h->perm) TRY(dalloc(h, &h->perm, ((size_t)std::max<int64_t>(h->cap, 1) + 16) * 4));
     sp.perm = h->perm;
-    k_fused_perm<T><<<h->ntiles, SP_BT, 0, s>>>(sp);
+    launch_early(k_fused_perm<T>, h->ntiles, SP_BT, s, sp);
     CKLAUNCH("k_fused_perm");
     h->lazy = true;
   }
