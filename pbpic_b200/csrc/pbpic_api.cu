@@ -1128,12 +1128,16 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
     A(&h->vals[b], capn * 4);
   }
   for (int k = 0; k < 6; ++k) A(&h->f[k], (size_t)pe * h->tsz);
-  for (int k = 0; k < 6; ++k) A(&h->f2[k], (size_t)pe * h->tsz);
+  const size_t plane_bytes = ((size_t)pe * h->tsz + 255) & ~(size_t)255;
+  A(&h->f2[0], 6 * plane_bytes);  // (one block for what is kept together: an allocation costs 0.1 ms)
+  for (int k = 1; k < 6 && r == PBPIC_OK; ++k) h->f2[k] = (char*)h->f2[0] + k * plane_bytes;
   A(&h->ng, (size_t)(c.mx + 1) * (c.my + 1) * 8 * h->tsz);
   if (h->mixed) A(&h->cg, (size_t)c.mx * c.my * 24 * h->tsz);
-  A(&h->jacc, (size_t)4 * pe * 8);
-  A(&h->jacc2, (size_t)4 * pe * 8);
-  A(&h->ticket, 16);
+  A(&h->jacc, (size_t)8 * pe * 8);
+  if (r == PBPIC_OK) h->jacc2 = (char*)h->jacc + (size_t)4 * pe * 8;
+  const size_t sync_bytes = 256 + (size_t)(CS_MAXCHUNKS + 1) * 8;
+  A(&h->ticket, sync_bytes);
+  if (r == PBPIC_OK) h->chunk_words = (unsigned long long*)((char*)h->ticket + 256);
   A(&h->counts, (size_t)(h->ncells + 1) * 4);
   A(&h->off, (size_t)(h->ncells + 1) * 4);
   A(&h->tile_off, (size_t)(h->ntiles + 1) * 4);
@@ -1153,7 +1157,6 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
   const int64_t sc = std::max({scan_scratch_ints(radix_hist_ints((int64_t)capn)), scan_scratch_ints(h->ncells + 1),
                                nchunks + 1 + scan_scratch_ints(nchunks)});
   A(&h->scan_scratch, (size_t)sc * 4);
-  A(&h->chunk_words, (size_t)(CS_MAXCHUNKS + 1) * 8);
   A(&h->rho, (size_t)pe * 8);
   A(&h->dscalar, 64);  // scalars of the diagnostics (up to 4 doubles)
   if (r != PBPIC_OK) {
@@ -1167,8 +1170,7 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
   cudaMemset(h->counts, 0, (size_t)(h->ncells + 1) * 4);
   cudaMemset(h->off, 0, (size_t)(h->ncells + 1) * 4);
   cudaMemset(h->status, 0, 16);
-  cudaMemset(h->ticket, 0, 16);
-  cudaMemset(h->chunk_words, 0, (size_t)(CS_MAXCHUNKS + 1) * 8);
+  cudaMemset(h->ticket, 0, sync_bytes);
   if (ensure_hist(h, 64) != PBPIC_OK || set_unsorted_tiles(h) != PBPIC_OK) {
     pbpic_destroy(h);
     return PBPIC_ENOMEM;
