@@ -36,9 +36,9 @@ METRIC = "particle-steps/s on 1 B200: FP32 mixed vs FP64 plain at stated energy 
 # DRAM bytes per particle of one launch of the mixed-form push as benchmarked (read + write: the
 # state read through the sort's permutation, the permutation itself, the state written in cell
 # order), from the ncu capture of the 512x256 sheet summarised in
-# profiles/k_push_fp32_harris_512x256_ppc100.txt; traffic grows in proportion to the particles.
-PUSH_DRAM_BYTES_PER_PARTICLE = 61.2
-PUSH_KERNEL = "k_push<float,true,true,false,true>"
+# profiles/k_push_cells_fp32_harris_512x256_ppc100.txt; traffic grows in proportion to the particles.
+PUSH_DRAM_BYTES_PER_PARTICLE = 52.4
+PUSH_KERNEL = "k_push_cells<float,32,true,false>"
 UNIT = "particle-steps/s"
 
 
@@ -139,7 +139,7 @@ class ClockSampler:
         self.active = False
         try:
             self.p = subprocess.Popen(["nvidia-smi", "-i", str(index), f"--query-gpu={self.FIELDS}",
-                                       "--format=csv,noheader,nounits", "-lms", "50"],
+                                       "--format=csv,noheader,nounits", "-lms", "20"],
                                       stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.t = threading.Thread(target=self._read, daemon=True)
             self.t.start()
@@ -206,8 +206,7 @@ def run_gpu(args, ranks):
             torch.cuda.synchronize()
             K = args.steps
             launches0 = pbpic_b200.kernel_launches()
-            if prec == "fp32":
-                sampler.active = True
+            sampler.active = True  # (both forms: 20 FP32 steps are over in 30 ms)
             start = torch.cuda.Event(enable_timing=True)
             end = torch.cuda.Event(enable_timing=True)
             start.record(stream)
