@@ -532,8 +532,15 @@ static __global__ void __launch_bounds__(CS_BT) k_fused_tables(FusedSortParams a
   }
   // (not earlier: the ranking's waiting blocks would take the field solve's places, 68 -> 78 us a step of sparse beams)
   cudaTriggerProgrammaticLaunchCompletion();
-  // every block has read the totals once all are done: the last one clears them
-  if (t == 0) done = (int)atomicAdd(&words[0], 1ull);
+  // Every block has left its total and read the others' once all are counted: the last one clears them. The
+  // barrier above puts this block's store and reads before thread 0's first fence, and the fences put
+  // them before its count and every other block's before the clearing: a total that
+  // landed after the zero of its word would be taken for one of the next launch.
+  if (t == 0) {
+    __threadfence();
+    done = (int)atomicAdd(&words[0], 1ull);
+    __threadfence();
+  }
   __syncthreads();
   if (done != (int)gridDim.x - 1) return;
   for (int k = t; k < (int)gridDim.x + 1; k += CS_BT) words[k] = 0ull;
