@@ -398,12 +398,14 @@ __device__ __forceinline__ CellEntries cell_entries(const FusedSortParams& a, in
   return e;
 }
 
+// (tilecnt by plain loads, not __ldg: k_fused_tables starts while the push still writes it, so that it is not
+// read-only for the kernel's lifetime, and a non-coherent load may be moved above the wait for the push.)
 __device__ __forceinline__ int32_t fused_count(const FusedSortParams& a, int c) {
   const int cx = c / a.my, cy = c - cx * a.my;
   const CellEntries e = cell_entries(a, cx, cy);
   int32_t v[9], s = 0;
 #pragma unroll
-  for (int k = 0; k < 9; ++k) v[k] = e.row[k % 3] >= 0 ? __ldg(a.tilecnt + e.col[k / 3] + e.row[k % 3]) : 0;
+  for (int k = 0; k < 9; ++k) v[k] = e.row[k % 3] >= 0 ? a.tilecnt[e.col[k / 3] + e.row[k % 3]] : 0;
 #pragma unroll
   for (int k = 0; k < 9; ++k) s += v[k];
   return s;
@@ -415,7 +417,7 @@ __device__ __forceinline__ void fused_slots(const FusedSortParams& a, int c, int
   const CellEntries e = cell_entries(a, cx, cy);
   int32_t v[9];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) v[k] = e.row[k % 3] >= 0 ? __ldg(a.tilecnt + e.col[k / 3] + e.row[k % 3]) : 0;
+  for (int k = 0; k < 9; ++k) v[k] = e.row[k % 3] >= 0 ? a.tilecnt[e.col[k / 3] + e.row[k % 3]] : 0;
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     if (e.row[k % 3] >= 0) a.base[e.col[k / 3] + e.row[k % 3]] = o;

@@ -78,3 +78,26 @@ def test_chunk_totals_are_clear_after_every_launch():
     assert not left_over(steps)
     at = steps.index("A")  # the fence after the count: nothing of the clearing is issued ahead of it
     assert steps[at - 1] == "F" and steps[at + 1] == "F"
+
+
+def test_early_launches_load_coherently():
+    """A kernel that starts under the one before it (launch_early) must not read through the
+    non-coherent path, which is for memory that nothing writes while the kernel lives."""
+    api = source("pbpic_api.cu")
+    early = set(re.findall(r"launch_early\((k_\w+)", api))
+    assert early == {"k_fused_tables", "k_fused_perm"}
+    bodies = {}
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith(".cuh"):
+            for k, body in functions(source(name)).items():
+                bodies[k] = bodies.get(k, "") + body
+    reached, todo = set(), list(early)
+    while todo:  # the kernels and every device function they call
+        k = todo.pop()
+        if k not in reached:
+            reached.add(k)
+            todo += [c for c in re.findall(r"\b(\w+)\s*(?:<[^;<>()]*>)?\(", bodies[k]) if c in bodies]
+    assert {"chunk_counts", "chunk_tables", "fused_count", "fused_slots", "perm_tile"} <= reached
+    for k in reached:
+        assert "cudaGridDependencySynchronize" in bodies[k] or k not in early, k
+        assert not re.search(r"__ldg\(|\bldg_part\(|\.nc\b", bodies[k]), k
