@@ -15,9 +15,18 @@
 // the main pass their branch would run almost every time for one or two lanes.
 //
 // Mixed form's window: every value v (FP32, |v| below 2^15) is added in fixed point as
-// hi * 2^17 + lo to two 32-bit shared sums, which native shared atomics
-// update (see kernels_push.cuh); a tile of more than 32767 particles uses the
-// same memory as 64-bit sums.
+// hi * 2^16 + lo to two signed 32-bit shared sums, which native shared atomics
+// update; a tile of more than 32767 particles uses the same memory as 64-bit
+// sums. hi = v 2^16 rounded to nearest, so that both parts are exact and lo, |lo| <= 2^15, has
+// the rounding that the 64-bit sum would give v. With at most 32767 particles neither
+// sum can overflow. A particle takes part in at most two additions to an entry: a crosser's two segments can share a
+// node (jx when it leaves through a y face, jy through an x face), and a cell's
+// sums, one addition a chunk of at least one particle, hold jx and jy of the others only and jz and rho of all. So
+//   |sum of lo| <= 2 * 32767 * 2^15 < 2^31;
+//   |sum of hi| <= 32767 * (2^16 + 1) + rounding < 2^31,
+// since what a particle adds to an entry is at most 1 in all (a move of less than a cell, a speed below c, a
+// charge, each times a weight), each addition rounds by 1/2, and 32767 steps are left for the FP32 rounding.
+// (The split at 2^17 of kernels_push.cuh, with lo >= 0, holds for one addition a particle only.)
 //
 // What bounds it, and why this form (512x256 Harris sheet, 26.2 M particles): the tile
 // push of kernels_push.cuh takes 575 us, 14.7 warp instructions a
@@ -147,11 +156,11 @@ __device__ __forceinline__ void shared_add(unsigned addr, unsigned v) {
   asm volatile("red.shared.add.u32 [%0], %1;\n" ::"r"(addr), "r"(v) : "memory");
 }
 __device__ __forceinline__ void win_add(const CellsWin& w, int idx, float v) {
-  if (w.split) {  // v 2^32 = h 2^17 + l, h = floor(v 2^15); both parts are exact in FP32
-    const float s = __fmul_rn(v, 32768.0f);
-    const float f = floorf(s);
-    shared_add(w.hi + 4 * idx, (unsigned)(int)f);
-    shared_add(w.lo + 4 * idx, (unsigned)__float2int_rn(__fmul_rn(__fsub_rn(s, f), 131072.0f)));
+  if (w.split) {  // v 2^32 = h 2^16 + l, h = v 2^16 rounded; s - h and its product are exact
+    const float s = __fmul_rn(v, 65536.0f);
+    const float h = rintf(s);
+    shared_add(w.hi + 4 * idx, (unsigned)(int)h);
+    shared_add(w.lo + 4 * idx, (unsigned)__float2int_rn(__fmul_rn(__fsub_rn(s, h), 65536.0f)));
   } else {
     asm volatile("red.shared.add.u64 [%0], %1;\n" ::"r"(w.lo + 8 * idx), "l"(to_acc<float, true>(v)) : "memory");
   }
@@ -640,7 +649,7 @@ __device__ __forceinline__ void push_cells(const PushParams<T>& a, const int t, 
   if constexpr (F32) {
     long long* gacc = reinterpret_cast<long long*>(a.jacc);
     for (int e = threadIdx.x; e < 16 * w.WR; e += PC_THREADS) {
-      const long long val = w.split ? ((long long)hi[e] << 17) + (long long)lo[e] : reinterpret_cast<const long long*>(lo)[e];
+      const long long val = w.split ? (long long)hi[e] * 65536 + (int)lo[e] : reinterpret_cast<const long long*>(lo)[e];
       if (val == 0) continue;
       const int cmp = e / (4 * w.WR), r = e - cmp * 4 * w.WR, wx = r / w.WR, wy = r - wx * w.WR;
       long long gi;
