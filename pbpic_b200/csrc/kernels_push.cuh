@@ -106,8 +106,7 @@ __device__ __forceinline__ Node6<double> load_node_staged(const double* g) {
 // ez bx by bz, one aligned 16-byte group each), the bilinear coefficients
 // (A, B, C, D) of the field over the cell, f(x, y) = A + B x + C y + D x y for
 // the in-cell offsets x, y in [-1/2, 1/2): the same bilinear interpolation of
-// the 4 nodes as pic2d.f90:948-963, 3 FMAs per field. PBPIC_CELL_COEF = 0
-// (device_common.cuh) keeps the 4 nodes themselves instead.
+// the 4 nodes as pic2d.f90:948-963, 3 FMAs per field.
 
 struct CellCoef {
   float4 f[6];
@@ -125,18 +124,6 @@ __device__ __forceinline__ void load_coef_staged(const float* r, CellCoef& c) {
 }
 __device__ __forceinline__ float coef_at(const float4& q, float x, float y) {
   return __fmaf_rn(__fmaf_rn(q.w, x, q.z), y, __fmaf_rn(q.y, x, q.x));
-}
-
-// The 4 gather nodes of a cell from its record: n00, n01, n10, n11, each ex ey
-// ez bx by bz (6 aligned 16-byte loads from one address).
-__device__ __forceinline__ void load_cell(const float* r, Node6<float>& n00, Node6<float>& n01, Node6<float>& n10,
-                                          Node6<float>& n11) {
-  const float4* q = reinterpret_cast<const float4*>(r);
-  const float4 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), d = __ldg(q + 3), e = __ldg(q + 4), f = __ldg(q + 5);
-  n00 = Node6<float>{a.x, a.y, a.z, a.w, b.x, b.y};
-  n01 = Node6<float>{b.z, b.w, c.x, c.y, c.z, c.w};
-  n10 = Node6<float>{d.x, d.y, d.z, d.w, e.x, e.y};
-  n11 = Node6<float>{e.z, e.w, f.x, f.y, f.z, f.w};
 }
 
 __device__ __forceinline__ void ld4(const uint32_t* p, uint32_t (&v)[4]) {
@@ -750,7 +737,7 @@ __device__ __forceinline__ TileWin<T, MIXED> tile_begin(const PushParams<T>& a, 
   w.y1 = min(w.y0 + w.TY, a.my);
   w.stg = reinterpret_cast<const T*>(smem_raw + (MIXED ? push_rec_offset(w.TY) : push_node_offset(w.TY)));
   w.mbar = mbar;
-  if constexpr (MIXED && PBPIC_CELL_COEF && PBPIC_PUSH_STAGE_RECS) {
+  if constexpr (MIXED && PBPIC_PUSH_STAGE_RECS) {
     // the records of cells (ixt, y0..y1-1) are contiguous: one copy of 96 B per row
     if (threadIdx.x == 0) {
       const unsigned bytes = (unsigned)(w.y1 - w.y0) * 96u;
@@ -908,7 +895,7 @@ template <class T, bool MIXED, bool HIST, int G, bool COMPAT = true, bool GATHER
 __device__ __forceinline__ void push_tile(const PushParams<T>& a, const int t, PushSmem<T, MIXED>& sm,
                                           unsigned char* smem_raw, unsigned parity) {
   constexpr int PT = 4 * G;  // particles per thread per pass
-  constexpr bool STAGED = MIXED ? (PBPIC_CELL_COEF && PBPIC_PUSH_STAGE_RECS) : PBPIC_PUSH_STAGE_NODES;
+  constexpr bool STAGED = MIXED ? PBPIC_PUSH_STAGE_RECS : PBPIC_PUSH_STAGE_NODES;
   const TileWin<T, MIXED> tw = tile_begin<T, MIXED, HIST>(a, t, smem_raw, &sm.mbar);
   const int TY = tw.TY, WR = tw.WR, ixt = tw.ixt, y0 = tw.y0, y1 = tw.y1;
   bool staged = false;  // this thread reads the tile's records from shared memory
@@ -1013,10 +1000,8 @@ __device__ __forceinline__ void push_tile(const PushParams<T>& a, const int t, P
             const int r = iy - y0;
             if (staged && inwin) load_coef_staged(tw.stg + r * 24, cc);
             else load_coef(a.cg + ((long long)ix * a.my + iy) * 24, cc);
-          } else if constexpr (MIXED && PBPIC_CELL_COEF) {
-            load_coef(a.cg + ((long long)ix * a.my + iy) * 24, cc);
           } else if constexpr (MIXED) {
-            load_cell(a.cg + ((long long)ix * a.my + iy) * 24, n00, n01, n10, n11);
+            load_coef(a.cg + ((long long)ix * a.my + iy) * 24, cc);
           } else if (STAGED && staged && inwin) {
             // FP64 from the tile's staged node columns
             const T* s00 = tw.stg + (iy - y0) * 8;
@@ -1036,7 +1021,7 @@ __device__ __forceinline__ void push_tile(const PushParams<T>& a, const int t, P
           cache_cell = cid;
         }
         Pushed<T> o;
-        if constexpr (MIXED && PBPIC_CELL_COEF)
+        if constexpr (MIXED)
           push_one_coef<COMPAT>(a, sp, ix, iy, px[0], py[0], pux[0], puy[0], puz[0], cc, o);
         else
           push_one<T, MIXED, COMPAT>(a, sp, ix, iy, px[0], py[0], pux[0], puy[0], puz[0], n00, n01, n10, n11, o);

@@ -317,7 +317,7 @@ size_t push_smem_bytes(int ty, bool mixed) {
     if (PBPIC_PUSH_STAGE_NODES) return push_node_offset(ty) + (size_t)2 * (ty + 1) * 64;  // + staged node columns
     return push_first_offset(ty) + (size_t)(PushThreads<double>::value / 32) * 17 * 33 * sizeof(double);
   }
-  if (PBPIC_CELL_COEF && PBPIC_PUSH_STAGE_RECS) return push_rec_offset(ty) + (size_t)ty * 96;  // + staged records
+  if (PBPIC_PUSH_STAGE_RECS) return push_rec_offset(ty) + (size_t)ty * 96;  // + staged records
   return (size_t)16 * (ty + 3) * 8 + (size_t)3 * (ty + 2) * 4 + (size_t)16 * (ty + 3) * 4;
 }
 
