@@ -48,22 +48,25 @@ struct DiffState {
   uint32_t* cell;
   Comps<T> c;      // dx dy ux uy as one record, uz
   int32_t* id;     // index in load order (pairs: 2k ion, 2k+1 electron)
-  int32_t* perm;   // position in cell order -> element
+  int32_t* perm;   // position in cell order -> element, bit 31 for a background particle (perm_entry)
 };
+constexpr int32_t PERM_ELEM = 0x7fffffff;
+__device__ __forceinline__ int32_t perm_entry(int64_t e, int32_t id, int64_t nsheet) {
+  return (int32_t)e | ((id >> 1) < nsheet ? 0 : (int32_t)0x80000000);
+}
 
 template <class T>
 struct DiffParams {
   PushParams<T> push;     // constants, geometry, the node grid of step n and the current
   int64_t n;              // particles
-  int64_t nsheet;         // pairs k < nsheet are sheet particles (weight 1)
-  double omega_bg;        // weight of background particles
+  double omega_bg;        // weight of background particles (of the sheet's: 1)
   double in0;             // current normalisation
-  DiffState<T> in, out;   // states before and after the step (out: forward only)
+  DiffState<T> in, out;   // states before and after the step (out: forward only, cell null: not wanted)
   int32_t* rank;          // forward: each new element's rank in its cell
   int32_t* counts;        // and the cells' counts (0 on entry)
-  Comps<T> lam_in;        // adjoint of the state after the step
+  Comps<T> lam_in;        // adjoint of the state after the step (null: zero)
   const int32_t* remap;   // null, or the element of each particle (by id) in lam_in's order
-  Comps<T> lam_out;       // adjoint of the state before the step
+  Comps<T> lam_out;       // adjoint of the state before the step; may be in.c itself
   const double* jbar;     // adjoint of the normalised current, 3 planes of mx x S
   double* gbar;           // adjoint of the node fields (mx+1) x (my+1) x 8
   double* domega;         // d loss / d omega_bg (one double)
@@ -126,17 +129,17 @@ __global__ void __launch_bounds__(DT) k_dpush(DiffParams<T> a) {
   const PushParams<T>& pp = a.push;
   const int64_t j = (int64_t)blockIdx.x * DT + threadIdx.x;
   const bool ok = j < a.n;
-  const int e = ok ? a.in.perm[j] : 0;
+  const int32_t pe = ok ? a.in.perm[j] : 0;
+  const int e = pe & PERM_ELEM;
   const uint32_t w = a.in.cell[e];
   const int sp = cw_sp(w), ix = cw_ix(w), iy = cw_iy(w);
-  const int32_t id = a.in.id[e];
   const T* g00 = pp.ng + ((long long)ix * (pp.my + 1) + iy) * 8;
   const T* g10 = g00 + (long long)(pp.my + 1) * 8;
   const Node6<T> n00 = load_node(g00), n01 = load_node(g00 + 8), n10 = load_node(g10), n11 = load_node(g10 + 8);
   Pushed<T> o;
   const P5<T> q = ldg_part(a.in.c, e);
   push_one<T, false>(pp, sp, ix, iy, q.dx, q.dy, q.ux, q.uy, q.uz, n00, n01, n10, n11, o);
-  const double om = !ok ? 0.0 : ((id >> 1) < a.nsheet ? 1.0 : a.omega_bg);
+  const double om = !ok ? 0.0 : (pe >= 0 ? 1.0 : a.omega_bg);
   double t[12];
 #pragma unroll
   for (int k = 0; k < 12; ++k) {
@@ -180,10 +183,11 @@ __global__ void __launch_bounds__(DT) k_dpush(DiffParams<T> a) {
     const int cx = rk / pp.my, cy = rk - cx * pp.my;
     put(kc, cx, cy, kx, ky, sum);
   });
+  if (!a.out.cell) return;  // (the whole grid)
   if (ok) {
     a.out.cell[j] = o.cw;
     put_part(a.out.c, j, P5<T>{o.dx, o.dy, o.ux, o.uy, o.uz});
-    a.out.id[j] = id;
+    a.out.id[j] = a.in.id[e];
   }
   const int32_t r = count_in_cell(a.counts, ok ? cw_ix(o.cw) * pp.my + cw_iy(o.cw) : -1);
   if (ok) a.rank[j] = r;
@@ -208,16 +212,17 @@ __global__ void __launch_bounds__(DT, DADJ_MINBLOCKS) k_dadjoint(DiffParams<T> a
   double domega = 0.0;
   const int64_t j = (int64_t)blockIdx.x * DT + threadIdx.x;
   const bool ok = j < a.n;
-  const int e = ok ? a.in.perm[j] : 0;
+  const int32_t pe = ok ? a.in.perm[j] : 0;
+  const int e = pe & PERM_ELEM;
   const uint32_t w = a.in.cell[e];
   const int sp = cw_sp(w), ix = cw_ix(w), iy = cw_iy(w);
-  const int32_t id = a.in.id[e];
-  const bool sheet = (id >> 1) < a.nsheet;
-  const int64_t p = a.remap ? a.remap[id] : (ok ? j : 0);  // the particle in the state after the step
+  const bool sheet = pe >= 0;
+  const int64_t p = !ok ? 0 : (a.remap ? a.remap[a.in.id[e]] : j);  // the particle in the state after the step
   const T* g00 = pp.ng + ((long long)ix * (pp.my + 1) + iy) * 8;
   const T* g10 = g00 + (long long)(pp.my + 1) * 8;
   const Node6<T> n00 = load_node(g00), n01 = load_node(g00 + 8), n10 = load_node(g10), n11 = load_node(g10 + 8);
-  const P5<T> q = ldg_part(a.in.c, e), l1 = ldg_part(a.lam_in, p);
+  // (in.c by plain loads, by the element's own thread only: lam_out may take its place)
+  const P5<T> q = ok ? get_part(a.in.c, e) : P5<T>{}, l1 = a.lam_in.q ? ldg_part(a.lam_in, p) : P5<T>{};
   const T px = q.dx, py = q.dy, pux = q.ux, puy = q.uy, puz = q.uz;
   Pushed<T> o;  // the forward push, for the branch decisions and the deposit terms
   push_one<T, false>(pp, sp, ix, iy, px, py, pux, puy, puz, n00, n01, n10, n11, o);
@@ -450,11 +455,11 @@ static __global__ void k_diff_psi(pic::FieldInit f, int S, const double* bx, con
   if (threadIdx.x == 0) atomicAdd(out, s);
 }
 // The permutation of a state from its elements' ranks in their cells.
-static __global__ void k_diff_perm(const uint32_t* cell, const int32_t* rank, const int32_t* off, int64_t n, int my,
-                                   int32_t* perm) {
+static __global__ void k_diff_perm(const uint32_t* cell, const int32_t* id, int64_t nsheet, const int32_t* rank,
+                                   const int32_t* off, int64_t n, int my, int32_t* perm) {
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t w = cell[e];
-    perm[off[(int64_t)cw_ix(w) * my + cw_iy(w)] + rank[e]] = (int32_t)e;
+    perm[off[(int64_t)cw_ix(w) * my + cw_iy(w)] + rank[e]] = perm_entry(e, id[e], nsheet);
   }
 }
 // Element of each particle (by id).
@@ -470,15 +475,15 @@ static __global__ void k_diff_rank(const uint32_t* cell, int64_t n, int my, int3
   if (e < n) rank[e] = r;
 }
 template <class T>
-__global__ void k_diff_move(const uint32_t* cell, Comps<T> in, const int32_t* rank, const int32_t* off, int64_t n,
-                            int my, DiffState<T> out) {
+__global__ void k_diff_move(const uint32_t* cell, Comps<T> in, int64_t nsheet, const int32_t* rank, const int32_t* off,
+                            int64_t n, int my, DiffState<T> out) {
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t w = cell[e];
     const int64_t d = (int64_t)off[(int64_t)cw_ix(w) * my + cw_iy(w)] + rank[e];
     out.cell[d] = w;
     put_part(out.c, d, get_part(in, e));
     out.id[d] = (int32_t)e;
-    out.perm[d] = (int32_t)d;
+    out.perm[d] = perm_entry(d, (int32_t)e, nsheet);
   }
 }
 

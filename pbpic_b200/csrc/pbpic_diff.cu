@@ -47,9 +47,8 @@ int grid_of(int64_t n, int maxblocks = 148 * 8) {
 
 // One stored state: particles and Yee fields.
 struct Slot {
-  void* p = nullptr;   // records of 4 T and uz (T), cell words, ids and permutation (4 B each)
-  void* f = nullptr;   // 6 planes of T
-  void* ng = nullptr;  // node grid of those fields
+  void* p = nullptr;  // records of 4 T and uz (T), cell words and ids (a checkpoint) or the permutation (4 B each)
+  void* f = nullptr;  // 6 planes of T
 };
 
 }  // namespace
@@ -62,15 +61,23 @@ struct pbpic_diff {
   int64_t n = 0, npairs = 0, nsheet = 0;
   double dx = 0, dy = 0, dt = 0, cva = 0, in0 = 0;
   int nseg = 0;
+  // The states that exist at once. What a state holds beside its particles and fields is kept only where
+  // it cannot be had again: a checkpoint's permutation and every node grid are formed when the
+  // state is opened, a state's ids only where the order is left (checkpoints; the two newest states), whether a
+  // particle is background in its permutation entry, and a state's adjoint takes its particles' place.
   std::vector<Slot> ck;   // checkpoints: state at steps 0, K, 2K, ...
-  std::vector<Slot> seg;  // recomputed states of one segment (K + 1)
-  Slot work[2];           // running states of a forward run
+  std::vector<Slot> seg;  // [1..K-1]: the states between two checkpoints, of the segment at work
+  Slot fin;               // magnetic loss: fields of the last state (no push reads its particles)
+  int32_t* ckperm = nullptr;                // the open checkpoint's permutation
+  int32_t* ids[2] = {nullptr, nullptr};     // ids of the newest even and odd state of the segment
+  void* ng = nullptr;                       // node grid of the state before step ng_at
+  int ng_at = -1;
   void* jacc[2] = {nullptr, nullptr};  // 4 planes of 8-byte accumulators; [0] is clear before a push
   double* fe_part = nullptr;
   int nfe = 0;
   int32_t *rank = nullptr, *counts = nullptr, *off = nullptr, *sums = nullptr;  // cell order of a new state
   bool last_seg = false;  // seg holds the states of the forward run's last segment
-  void* lam[2] = {nullptr, nullptr};  // particle adjoints: records of 4 T, then uz
+  void* lam[2] = {nullptr, nullptr};  // particle adjoints of a checkpoint (the second for K = 1): records of 4 T, then uz
   double* fbar = nullptr;  // 6 adjoint planes (ex ey ez bx by bz)
   double* jbar = nullptr;  // 3 planes
   double* gbar = nullptr;  // node adjoint
@@ -96,7 +103,7 @@ int dmalloc(pbpic_diff* d, void** p, size_t bytes) {
   return PBPIC_OK;
 }
 
-size_t part_bytes(const pbpic_diff* d) { return (size_t)d->n * (12 + 5 * d->tsz); }
+size_t part_bytes(const pbpic_diff* d) { return (size_t)d->n * (8 + 5 * d->tsz); }
 size_t field_bytes(const pbpic_diff* d) { return (size_t)6 * d->mx * d->S * d->tsz; }
 size_t node_bytes(const pbpic_diff* d) { return (size_t)(d->mx + 1) * (d->my + 1) * 8 * d->tsz; }
 int64_t plane(const pbpic_diff* d) { return (int64_t)d->mx * d->S; }
@@ -108,13 +115,24 @@ struct View {
 };
 
 template <class T>
-View<T> view(const pbpic_diff* d, const Slot& s) {
-  View<T> v;
-  T* base = (T*)s.p;
-  v.p.c = Comps<T>{base, base + (size_t)4 * d->n};
-  v.p.cell = (uint32_t*)(base + (size_t)5 * d->n);
-  v.p.id = (int32_t*)(v.p.cell + d->n);
-  v.p.perm = v.p.id + d->n;
+Comps<T> comps(const pbpic_diff* d, void* p) {
+  return Comps<T>{(T*)p, (T*)p + (size_t)4 * d->n};
+}
+
+// The state before step it (it = nsteps: the last state's fields).
+template <class T>
+View<T> state(const pbpic_diff* d, int it) {
+  const int K = d->cfg.checkpoint_every;
+  const bool final = it == d->cfg.nsteps, ck = !final && it % K == 0;
+  const Slot& s = final ? d->fin : (ck ? d->ck[it / K] : d->seg[it % K]);
+  View<T> v{};
+  if (!final) {
+    v.p.c = comps<T>(d, s.p);
+    v.p.cell = (uint32_t*)((T*)s.p + (size_t)5 * d->n);
+    int32_t* last = (int32_t*)(v.p.cell + d->n);
+    v.p.id = ck ? last : d->ids[it & 1];
+    v.p.perm = ck ? d->ckperm : last;
+  }
   for (int k = 0; k < 6; ++k) v.f[k] = (T*)s.f + (size_t)k * plane(d);
   return v;
 }
@@ -139,7 +157,7 @@ double urel(double v) { return v / sqrt(1.0 - v * v); }
 double durel(double v) { return 1.0 / pow(1.0 - v * v, 1.5); }
 
 template <class T>
-PushParams<T> push_params(const pbpic_diff* d, const Slot& s) {
+PushParams<T> push_params(const pbpic_diff* d) {
   PushParams<T> p;
   memset(&p, 0, sizeof(p));
   p.mx = d->mx;
@@ -147,7 +165,7 @@ PushParams<T> push_params(const pbpic_diff* d, const Slot& s) {
   p.S = d->S;
   p.ybc = PBPIC_BC_CONDUCTING;
   p.compat = 0;
-  p.ng = (const T*)s.ng;
+  p.ng = (const T*)d->ng;
   p.cg = nullptr;  // the adjoint kernels gather from the node grid
   p.jacc = d->jacc[0];
   const T dt = (T)d->dt, mime = (T)d->cfg.mime, cva = (T)d->cva, dx = (T)d->dx, dy = (T)d->dy;
@@ -169,8 +187,7 @@ PushParams<T> push_params(const pbpic_diff* d, const Slot& s) {
 }
 
 template <class T>
-FieldParams<T> field_params(const pbpic_diff* d, const Slot& s) {
-  View<T> v = view<T>(d, s);
+FieldParams<T> field_params(const pbpic_diff* d, const View<T>& v) {
   FieldParams<T> a{};
   a.mx = d->mx;
   a.my = d->my;
@@ -189,7 +206,7 @@ FieldParams<T> field_params(const pbpic_diff* d, const Slot& s) {
   a.idy = T(1) / (T)d->dy;
   a.jacc = d->jacc[0];
   for (int k = 0; k < 4; ++k) a.jscale[k] = d->f32 ? d->in0 * FIX_INV : d->in0;
-  a.ng = (T*)s.ng;
+  a.ng = (T*)d->ng;
   a.cg = nullptr;
   a.fe_part = d->fe_part;
   return a;
@@ -204,10 +221,9 @@ double jdote_scale(const pbpic_diff* d) { return d->dt * d->cfg.mime / (d->cva *
 double jdote_jscale(const pbpic_diff* d) { return d->f32 ? d->in0 * FIX_INV : d->in0; }
 
 // The j.E loss of the step whose current is in `jacc` and whose starting
-// fields are the slot's; with jbar/fbar_e, its adjoint seeds.
+// fields are the state's; with jbar/fbar_e, its adjoint seeds.
 template <class T>
-int loss_jdote(pbpic_diff* d, const Slot& s, const void* jacc, double* loss, double* jbar, double* fbar_e) {
-  View<T> v = view<T>(d, s);
+int loss_jdote(pbpic_diff* d, const View<T>& v, const void* jacc, double* loss, double* jbar, double* fbar_e) {
   const int g = grid_of((int64_t)d->mx * (d->my + 1));
   if (d->f32)
     k_loss_jdote<T, long long><<<g, 256>>>(d->mx, d->my, d->S, PBPIC_BC_CONDUCTING, jacc, jdote_jscale(d), v.f[0],
@@ -219,12 +235,14 @@ int loss_jdote(pbpic_diff* d, const Slot& s, const void* jacc, double* loss, dou
   return PBPIC_OK;
 }
 
-// Node grid of a slot's fields into d->ng.
+// Node grid of the state before step it into d->ng.
 template <class T>
-int nodes(pbpic_diff* d, const Slot& s) {
-  FieldParams<T> a = field_params<T>(d, s);
+int nodes(pbpic_diff* d, int it) {
+  if (d->ng_at == it) return PBPIC_OK;
+  FieldParams<T> a = field_params<T>(d, state<T>(d, it));
   k_nodes<T><<<d->nfe, 256>>>(a);
   DLAUNCH("k_nodes");
+  d->ng_at = it;
   return PBPIC_OK;
 }
 
@@ -240,47 +258,65 @@ int cell_offsets(pbpic_diff* d) {
   return PBPIC_OK;
 }
 
-// One forward step from slot s to slot o; adds the step's loss to scal[0]. With
-// the j.E loss and `jkeep`, also keeps the step's current (3 planes) there.
+// Opens checkpoint `it`: its permutation and its node grid.
 template <class T>
-int step(pbpic_diff* d, const Slot& s, const Slot& o, double omega, void* jkeep = nullptr) {
-  View<T> vs = view<T>(d, s), vo = view<T>(d, o);
+int open_checkpoint(pbpic_diff* d, int it) {
+  const View<T> v = state<T>(d, it);
+  k_diff_rank<<<(unsigned)((d->n + 255) / 256), 256>>>(v.p.cell, d->n, d->my, d->counts, d->rank);
+  DLAUNCH("k_diff_rank");
+  DTRY(cell_offsets(d));
+  k_diff_perm<<<grid_of(d->n, 148 * 16), 256>>>(v.p.cell, v.p.id, d->nsheet, d->rank, d->off, d->n, d->my, v.p.perm);
+  DLAUNCH("k_diff_perm");
+  return nodes<T>(d, it);
+}
+
+// Step it, from the state before it (its node grid in d->ng) to o, whose node grid is then in d->ng; adds the
+// step's loss to scal[0]. With the j.E loss and `jkeep`, also keeps the step's current (3 planes)
+// there. An o without particles or without fields: those are not wanted.
+template <class T>
+int step(pbpic_diff* d, int it, const View<T>& o, double omega, void* jkeep = nullptr) {
+  const View<T> s = state<T>(d, it);
   DiffParams<T> dp;
   memset(&dp, 0, sizeof(dp));
-  dp.push = push_params<T>(d, s);
+  dp.push = push_params<T>(d);
   dp.n = d->n;
-  dp.nsheet = d->nsheet;
   dp.omega_bg = omega;
   dp.in0 = d->in0;
-  dp.in = vs.p;
-  dp.out = vo.p;
+  dp.in = s.p;
+  dp.out = o.p;
   dp.rank = d->rank;
   dp.counts = d->counts;
   k_dpush<T><<<(unsigned)((d->n + DT - 1) / DT), DT>>>(dp);
   DLAUNCH("k_dpush");
-  DTRY(cell_offsets(d));
-  k_diff_perm<<<grid_of(d->n, 148 * 16), 256>>>(vo.p.cell, d->rank, d->off, d->n, d->my, vo.p.perm);
-  DLAUNCH("k_diff_perm");
+  if (o.p.cell) {
+    DTRY(cell_offsets(d));
+    k_diff_perm<<<grid_of(d->n, 148 * 16), 256>>>(o.p.cell, o.p.id, d->nsheet, d->rank, d->off, d->n, d->my, o.p.perm);
+    DLAUNCH("k_diff_perm");
+  }
   const bool jdote = d->cfg.loss == PBPIC_LOSS_JDOTE;
   if (jdote) {
     DTRY(loss_jdote<T>(d, s, d->jacc[0], d->scal, nullptr, nullptr));
     if (jkeep) DCK(cudaMemcpyAsync(jkeep, d->jacc[0], (size_t)3 * plane(d) * 8, cudaMemcpyDeviceToDevice));
   }
+  if (!o.f[0]) {  // (the field solve would have left a clear current)
+    DCK(cudaMemsetAsync(d->jacc[0], 0, (size_t)4 * plane(d) * 8));
+    return PBPIC_OK;
+  }
   FieldParams<T> a = field_params<T>(d, s);
-  a.nex = vo.f[0];
-  a.ney = vo.f[1];
-  a.nez = vo.f[2];
-  a.nbx = vo.f[3];
-  a.nby = vo.f[4];
-  a.nbz = vo.f[5];
-  a.ng = (T*)o.ng;
+  a.nex = o.f[0];
+  a.ney = o.f[1];
+  a.nez = o.f[2];
+  a.nbx = o.f[3];
+  a.nby = o.f[4];
+  a.nbz = o.f[5];
   a.jnext = d->jacc[1];
   if (d->f32) k_field_step<T, long long><<<field_tiles(d->mx, d->my), FT>>>(a);
   else k_field_step<T, double><<<field_tiles(d->mx, d->my), FT>>>(a);
   DLAUNCH("k_field_step");
   std::swap(d->jacc[0], d->jacc[1]);
+  d->ng_at = it + 1;
   if (!jdote) {
-    k_loss_b<T><<<grid_of((int64_t)(d->mx + 1) * (d->my + 1)), 256>>>(d->mx, d->my, 1, (const T*)o.ng,
+    k_loss_b<T><<<grid_of((int64_t)(d->mx + 1) * (d->my + 1)), 256>>>(d->mx, d->my, 1, (const T*)d->ng,
                                                                        loss_scale(d), d->scal, nullptr);
     DLAUNCH("k_loss_b");
   }
@@ -322,20 +358,23 @@ int load(pbpic_diff* d, const pbpic_diff_params* prm) {
   L.udrift_i = urel(hs.udi);
   L.lambda = c.lambda;
   L.seed = c.seed;
-  // loaded in load order, then moved into cell order
-  View<T> v = view<T>(d, d->work[0]), v0 = view<T>(d, d->ck[0]);
-  k_load<T><<<(unsigned)((d->npairs + 255) / 256), 256>>>(L, d->npairs, 0, v.p.cell, v.p.c, nullptr);
+  // loaded in load order (where the adjoint and a state's ids go later), then moved into cell order
+  const Comps<T> c0 = comps<T>(d, d->lam[0]);
+  uint32_t* cell0 = (uint32_t*)d->ids[0];
+  const View<T> v = state<T>(d, 0);
+  k_load<T><<<(unsigned)((d->npairs + 255) / 256), 256>>>(L, d->npairs, 0, cell0, c0, nullptr);
   DLAUNCH("k_load");
   DCK(cudaMemsetAsync(d->counts, 0, (size_t)d->mx * d->my * 4));
   DCK(cudaMemsetAsync(d->jacc[0], 0, (size_t)4 * plane(d) * 8));
-  k_diff_rank<<<(unsigned)((d->n + 255) / 256), 256>>>(v.p.cell, d->n, d->my, d->counts, d->rank);
+  k_diff_rank<<<(unsigned)((d->n + 255) / 256), 256>>>(cell0, d->n, d->my, d->counts, d->rank);
   DLAUNCH("k_diff_rank");
   DTRY(cell_offsets(d));
-  k_diff_move<T><<<grid_of(d->n, 148 * 16), 256>>>(v.p.cell, v.p.c, d->rank, d->off, d->n, d->my, v0.p);
+  k_diff_move<T><<<grid_of(d->n, 148 * 16), 256>>>(cell0, c0, d->nsheet, d->rank, d->off, d->n, d->my, v.p);
   DLAUNCH("k_diff_move");
-  k_diff_fields<T><<<grid_of(plane(d)), 256>>>(field_init(d, prm->psi0), d->S, (T*)d->ck[0].f);
+  k_diff_fields<T><<<grid_of(plane(d)), 256>>>(field_init(d, prm->psi0), d->S, v.f[0]);
   DLAUNCH("k_diff_fields");
-  return nodes<T>(d, d->ck[0]);
+  d->ng_at = -1;
+  return nodes<T>(d, 0);
 }
 
 template <class T>
@@ -347,14 +386,11 @@ int forward(pbpic_diff* d, const pbpic_diff_params* prm, double* loss) {
   const int last0 = (d->nseg - 1) * K;  // first step of the last segment, whose states stay for the adjoint
   const double omega = prm->nb / d->cfg.nb0;
   const size_t jbytes = (size_t)3 * plane(d) * 8;
-  // the state before step it: a checkpoint, a kept state of the last segment or a running state
-  auto slot = [&](int it) -> const Slot& {
-    if (it % K == 0 && it / K < d->nseg) return d->ck[it / K];
-    return it > last0 ? d->seg[it - last0] : d->work[it & 1];
-  };
   for (int it = 0; it < N; ++it) {
     const bool keep = it >= last0 && d->jseg;
-    DTRY(step<T>(d, slot(it), slot(it + 1), omega, keep ? (char*)d->jseg + (it - last0) * jbytes : nullptr));
+    // (the j.E loss of the last step ends with its current)
+    const View<T> o = it + 1 == N && d->jseg ? View<T>{} : state<T>(d, it + 1);
+    DTRY(step<T>(d, it, o, omega, keep ? (char*)d->jseg + (it - last0) * jbytes : nullptr));
   }
   DCK(cudaMemcpy(loss, d->scal, sizeof(double), cudaMemcpyDeviceToHost));
   d->last = *prm;
@@ -394,18 +430,17 @@ int backward(pbpic_diff* d, double grad[3]) {
   const size_t nodes_bytes = (size_t)(d->mx + 1) * (d->my + 1) * 8 * sizeof(double);
   const bool jdote = d->cfg.loss == PBPIC_LOSS_JDOTE;
   const size_t jbytes = (size_t)3 * pl * 8;
-  DCK(cudaMemset(d->lam[0], 0, (size_t)5 * d->n * d->tsz));
-  auto lam = [&](int b) { return Comps<T>{(T*)d->lam[b], (T*)d->lam[b] + (size_t)4 * d->n}; };
   DCK(cudaMemset(d->fbar, 0, (size_t)6 * pl * sizeof(double)));
   DCK(cudaMemset(d->gbar, 0, nodes_bytes));
   DCK(cudaMemset(d->scal + 1, 0, 3 * sizeof(double)));
-  int cur = 0;
+  Comps<T> lam{nullptr, nullptr};  // adjoint of the state after the step (none: zero), in its order
+  int buf = 0;
   AdjField af = adj_field(d);
   const int gf = grid_of((int64_t)d->mx * (d->my + 1));
   const int gn = grid_of((int64_t)(d->mx + 1) * (d->my + 1));
-  // magnetic loss of a state: the seed of its node adjoint
-  auto seed = [&](const Slot& s) -> int {
-    k_loss_b<T><<<gn, 256>>>(d->mx, d->my, 1, (const T*)s.ng, loss_scale(d), nullptr, d->gbar);
+  // magnetic loss of the state whose node grid is in d->ng: the seed of its node adjoint
+  auto seed = [&]() -> int {
+    k_loss_b<T><<<gn, 256>>>(d->mx, d->my, 1, (const T*)d->ng, loss_scale(d), nullptr, d->gbar);
     DLAUNCH("k_loss_b");
     return PBPIC_OK;
   };
@@ -413,16 +448,25 @@ int backward(pbpic_diff* d, double grad[3]) {
   d->last_seg = false;  // (the segments before it are recomputed into its place)
   for (int sg = d->nseg - 1; sg >= 0; --sg) {
     const int s0 = sg * K, s1 = std::min(N, s0 + K);
-    auto state = [&](int it) -> const Slot& { return it == s0 ? d->ck[sg] : d->seg[it - s0]; };
-    if (!(resident && sg == d->nseg - 1))
-      for (int it = s0; it < s1; ++it)  // recompute the segment, keeping every state
-        DTRY(step<T>(d, state(it), state(it + 1), omega, jdote ? (char*)d->jseg + (it - s0) * jbytes : nullptr));
-    if (sg == d->nseg - 1 && !jdote) {  // the last state's loss
-      DTRY(seed(state(N)));
+    const bool tail = sg == d->nseg - 1;
+    if (!(resident && tail)) {  // recompute the segment, keeping every state
+      DTRY(open_checkpoint<T>(d, s0));
+      for (int it = s0; it < s1; ++it) {
+        // the state after the segment is not needed, its adjoint comes by particle: of the last step
+        // the j.E loss wants the current, the magnetic one the fields at the end of the run
+        const bool end = it + 1 == s1;
+        if (end && !tail && !jdote) break;
+        const View<T> o = end && jdote ? View<T>{} : state<T>(d, it + 1);
+        DTRY(step<T>(d, it, o, omega, jdote ? (char*)d->jseg + (it - s0) * jbytes : nullptr));
+      }
+    }
+    if (tail && !jdote) {  // the last state's loss
+      DTRY(seed());
       k_adj_nodes<<<gn, 256>>>(af, d->gbar);
       DLAUNCH("k_adj_nodes");
     }
     for (int it = s1 - 1; it >= s0; --it) {
+      const View<T> v = state<T>(d, it);
       // transposed field solve: B half step, E full step, B half step in reverse
       k_adj_bhalf<<<gf, 256>>>(af);
       DLAUNCH("k_adj_bhalf");
@@ -431,35 +475,40 @@ int backward(pbpic_diff* d, double grad[3]) {
       // j.E loss of step it: E (the step's start) into the current adjoint, the
       // step's current into the adjoint of that E
       if (jdote)
-        DTRY(loss_jdote<T>(d, state(it), (char*)d->jseg + (it - s0) * jbytes, nullptr, d->jbar, d->fbar));
+        DTRY(loss_jdote<T>(d, v, (char*)d->jseg + (it - s0) * jbytes, nullptr, d->jbar, d->fbar));
       k_adj_bhalf<<<gf, 256>>>(af);
       DLAUNCH("k_adj_bhalf");
       // particle adjoint of the push of step it
+      DTRY(nodes<T>(d, it));
       DiffParams<T> dp;
       memset(&dp, 0, sizeof(dp));
-      dp.push = push_params<T>(d, state(it));
+      dp.push = push_params<T>(d);
       dp.n = d->n;
-      dp.nsheet = d->nsheet;
       dp.omega_bg = omega;
       dp.in0 = d->in0;
-      dp.in = view<T>(d, state(it)).p;
-      if (it == s1 - 1 && sg < d->nseg - 1) {  // lam comes in the order of the next checkpoint
-        k_diff_inverse<<<grid_of(d->n, 148 * 16), 256>>>(view<T>(d, d->ck[sg + 1]).p.id, d->n, d->rank);
+      dp.in = v.p;
+      if (it == s1 - 1 && !tail) {  // lam comes in the order of the next checkpoint
+        k_diff_inverse<<<grid_of(d->n, 148 * 16), 256>>>(state<T>(d, s1).p.id, d->n, d->rank);
         DLAUNCH("k_diff_inverse");
         dp.remap = d->rank;
       }
-      dp.lam_in = lam(cur);
-      dp.lam_out = lam(1 - cur);
+      dp.lam_in = lam;
+      if (it > s0) {  // the state's adjoint in its particles' place: nothing reads them after this
+        dp.lam_out = v.p.c;
+      } else {  // a checkpoint stays as it is
+        dp.lam_out = comps<T>(d, d->lam[buf]);
+        if (K == 1) buf = 1 - buf;  // (the next step reads from the buffer that this one wrote)
+      }
+      lam = dp.lam_out;
       dp.jbar = d->jbar;
       dp.gbar = d->gbar;
       dp.domega = d->scal + 1;
       k_dadjoint<T><<<(unsigned)((d->n + DT - 1) / DT), DT>>>(dp);
       DLAUNCH("k_dadjoint");
       // the state's own magnetic loss (none at the start), in the same transposed node average
-      if (!jdote && it > 0) DTRY(seed(state(it)));
+      if (!jdote && it > 0) DTRY(seed());
       k_adj_nodes<<<gn, 256>>>(af, d->gbar);
       DLAUNCH("k_adj_nodes");
-      cur = 1 - cur;
     }
   }
   // d loss / d tau through the loaded momenta (checkpoint 0 holds the initial state)
@@ -470,9 +519,9 @@ int backward(pbpic_diff* d, double grad[3]) {
     const double dvthi = dvthe * sqrt(tite / d->cfg.mime) + hs.vthe * 0.5 / sqrt(tite * d->cfg.mime);
     const double du = -1.0 / (d->cfg.lambda * d->cva);
     const double dudi_v = du / ((1.0 + tite) * (1.0 + tite)), dude_v = du / ((1.0 + tite) * (1.0 + tite));
-    View<T> v0 = view<T>(d, d->ck[0]);
+    const View<T> v0 = state<T>(d, 0);
     k_dtau<T><<<grid_of(d->n, 148 * 16), 256>>>(
-        d->n, d->nsheet, v0.p.id, v0.p.c, lam(cur), urel(hs.vthi), urel(hs.vthe), durel(hs.vthi) * dvthi, durel(hs.vthe) * dvthe,
+        d->n, d->nsheet, v0.p.id, v0.p.c, lam, urel(hs.vthi), urel(hs.vthe), durel(hs.vthi) * dvthi, durel(hs.vthe) * dvthe,
         urel(hs.udi), urel(hs.ude), durel(hs.udi) * dudi_v, durel(hs.ude) * dude_v, d->scal + 2);
     DLAUNCH("k_dtau");
   }
@@ -524,16 +573,18 @@ int pbpic_diff_create(const pbpic_diff_config* cfg, pbpic_diff** out) {
     if (r == PBPIC_OK) r = dmalloc(d, p, b);
   };
   d->ck.resize(d->nseg);
-  d->seg.resize(c.checkpoint_every + 1);
+  const int K = std::min(c.checkpoint_every, c.nsteps);
+  d->seg.resize(K);  // (a segment's first state is its checkpoint)
   auto slot = [&](Slot& s) {
     A(&s.p, part_bytes(d));
     A(&s.f, field_bytes(d));
-    A(&s.ng, node_bytes(d));
   };
   for (auto& s : d->ck) slot(s);
-  for (size_t k = 1; k < d->seg.size(); ++k) slot(d->seg[k]);  // (a segment's first state is its checkpoint)
-  slot(d->work[0]);
-  slot(d->work[1]);
+  for (int k = 1; k < K; ++k) slot(d->seg[k]);
+  if (c.loss == PBPIC_LOSS_MAGNETIC) A(&d->fin.f, field_bytes(d));
+  A((void**)&d->ckperm, (size_t)d->n * 4);
+  for (int b = 0; b < 2; ++b) A((void**)&d->ids[b], (size_t)d->n * 4);
+  A(&d->ng, node_bytes(d));
   for (int k = 0; k < 2; ++k) A(&d->jacc[k], (size_t)4 * plane(d) * 8);
   const int64_t nc = (int64_t)c.mx * c.my;
   A((void**)&d->rank, (size_t)d->n * 4);
@@ -542,12 +593,12 @@ int pbpic_diff_create(const pbpic_diff_config* cfg, pbpic_diff** out) {
   A((void**)&d->sums, (size_t)((nc + CS_TILE - 1) / CS_TILE + 1) * 4);
   d->nfe = grid_of((int64_t)(c.mx + 1) * (c.my + 1));
   A((void**)&d->fe_part, (size_t)std::max(d->nfe, field_tiles(c.mx, c.my)) * 2 * sizeof(double));
-  for (int b = 0; b < 2; ++b) A(&d->lam[b], (size_t)5 * d->n * d->tsz);
+  for (int b = 0; b < (c.checkpoint_every == 1 ? 2 : 1); ++b) A(&d->lam[b], (size_t)5 * d->n * d->tsz);
   A((void**)&d->fbar, (size_t)6 * plane(d) * sizeof(double));
   A((void**)&d->jbar, (size_t)3 * plane(d) * sizeof(double));
   A((void**)&d->gbar, (size_t)(c.mx + 1) * (c.my + 1) * 8 * sizeof(double));
   A((void**)&d->scal, 4 * sizeof(double));
-  if (c.loss == PBPIC_LOSS_JDOTE) A(&d->jseg, (size_t)c.checkpoint_every * 3 * plane(d) * 8);
+  if (c.loss == PBPIC_LOSS_JDOTE) A(&d->jseg, (size_t)K * 3 * plane(d) * 8);
   if (r != PBPIC_OK) {
     pbpic_diff_destroy(d);
     return r;
