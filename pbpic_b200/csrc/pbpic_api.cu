@@ -1114,9 +1114,13 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
   h->cap = c.capacity;
   const size_t capn = (size_t)std::max<int64_t>(c.capacity, 1);
   const int64_t pe = plane_elems(h);
-  int r = PBPIC_OK;
+  // Every array is a part of one block: an allocation and its release cost 0.1 ms or more each, and arrays of a megabyte take
+  // pages of their own.
+  std::vector<std::pair<void**, size_t>> parts;
+  size_t total = 0;
   auto A = [&](auto** p, size_t bytes) {
-    if (r == PBPIC_OK) r = dalloc(h, p, bytes);
+    parts.push_back({(void**)p, total});
+    total += (std::max<size_t>(bytes, 16) + 255) & ~(size_t)255;
   };
   for (int b = 0; b < 2; ++b) {
     // particle arrays carry 16 elements of padding: bulk copies read whole 16-byte units
@@ -1128,16 +1132,14 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
     A(&h->vals[b], capn * 4);
   }
   for (int k = 0; k < 6; ++k) A(&h->f[k], (size_t)pe * h->tsz);
-  const size_t plane_bytes = ((size_t)pe * h->tsz + 255) & ~(size_t)255;
-  A(&h->f2[0], 6 * plane_bytes);  // (one block for what is kept together: an allocation costs 0.1 ms)
-  for (int k = 1; k < 6 && r == PBPIC_OK; ++k) h->f2[k] = (char*)h->f2[0] + k * plane_bytes;
+  for (int k = 0; k < 6; ++k) A(&h->f2[k], (size_t)pe * h->tsz);
   A(&h->ng, (size_t)(c.mx + 1) * (c.my + 1) * 8 * h->tsz);
   if (h->mixed) A(&h->cg, (size_t)c.mx * c.my * 24 * h->tsz);
-  A(&h->jacc, (size_t)8 * pe * 8);
-  if (r == PBPIC_OK) h->jacc2 = (char*)h->jacc + (size_t)4 * pe * 8;
-  const size_t sync_bytes = 256 + (size_t)(CS_MAXCHUNKS + 1) * 8;
-  A(&h->ticket, sync_bytes);
-  if (r == PBPIC_OK) h->chunk_words = (unsigned long long*)((char*)h->ticket + 256);
+  A(&h->jacc, (size_t)4 * pe * 8);
+  A(&h->jacc2, (size_t)4 * pe * 8);
+  const size_t words_bytes = (size_t)(CS_MAXCHUNKS + 1) * 8;
+  A(&h->ticket, 16);
+  A(&h->chunk_words, words_bytes);
   A(&h->counts, (size_t)(h->ncells + 1) * 4);
   A(&h->off, (size_t)(h->ncells + 1) * 4);
   A(&h->tile_off, (size_t)(h->ntiles + 1) * 4);
@@ -1159,10 +1161,13 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
   A(&h->scan_scratch, (size_t)sc * 4);
   A(&h->rho, (size_t)pe * 8);
   A(&h->dscalar, 64);  // scalars of the diagnostics (up to 4 doubles)
+  char* block = nullptr;
+  const int r = dalloc(h, &block, total);
   if (r != PBPIC_OK) {
     pbpic_destroy(h);
     return r;
   }
+  for (const auto& [at, offset] : parts) *at = block + offset;
   for (int k = 0; k < 6; ++k) cudaMemset(h->f[k], 0, (size_t)pe * h->tsz);
   cudaMemset(h->ng, 0, (size_t)(c.mx + 1) * (c.my + 1) * 8 * h->tsz);
   if (h->cg) cudaMemset(h->cg, 0, (size_t)c.mx * c.my * 24 * h->tsz);
@@ -1170,7 +1175,8 @@ int pbpic_create(const pbpic_config* cfg, pbpic_handle** out) {
   cudaMemset(h->counts, 0, (size_t)(h->ncells + 1) * 4);
   cudaMemset(h->off, 0, (size_t)(h->ncells + 1) * 4);
   cudaMemset(h->status, 0, 16);
-  cudaMemset(h->ticket, 0, sync_bytes);
+  cudaMemset(h->ticket, 0, 16);
+  cudaMemset(h->chunk_words, 0, words_bytes);
   if (ensure_hist(h, 64) != PBPIC_OK || set_unsorted_tiles(h) != PBPIC_OK) {
     pbpic_destroy(h);
     return PBPIC_ENOMEM;
@@ -1670,10 +1676,10 @@ struct pbpic_batch {
 namespace {
 
 void dfree(pbpic_handle* h, void* p) {
-  if (!p) return;
-  cudaFree(p);
   auto it = std::find(h->allocs.begin(), h->allocs.end(), p);
-  if (it != h->allocs.end()) h->allocs.erase(it);
+  if (it == h->allocs.end()) return;  // none, or a part of the handle's block (pbpic_create)
+  cudaFree(p);
+  h->allocs.erase(it);
 }
 
 // Tile rows of a domain: ty, or the default for ty <= 0, capped so that the
