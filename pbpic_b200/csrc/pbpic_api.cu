@@ -375,12 +375,17 @@ Comps<T> C(pbpic_handle* h, int buf) {
 
 // Lanes per cell of the push cell by cell (kernels_push_cells.cuh: sorted input, no compat
 // switch, not the exact order), 0 for the tile push. By the domain's mean particles
-// per cell, uniform plasma on 512x256 cells, us per step.
-// Mixed, tile push / 16 lanes / 32 lanes: 8: 123 / 133 / 169; 12: 118 / 130 / 172;
-// 16: 133 / 136 / 168; 20: 153 / 136 / 168; 64: 269 / 197 / 230; 128: 446 / 309 / 320;
-// 200: 625 / 443 / 429 (a Harris sheet of 200: 670 / 458 / 439).
-// Plain, tile push / 32 lanes (16 lanes never better): 16: 187 / 234; 24: 231 / 251;
-// 32: 269 / 272; 64: 429 / 345; 128: 748 / 494; 180: 1007 / 625.
+// per cell; us per step of a uniform plasma on 512x256 cells, electrons of 0.1 c and of 0.3 c (where three times
+// as many particles leave their cell).
+// Mixed, tile push / 16 lanes / 32 lanes: 12: 109 / 126 / 161, 112 / 129 / 159; 16: 128 / 128 / 161, 130 / 128 / 161;
+// 18: 140 / 125 / 163, 144 / 130 / 163; 20: 146 / 130 / 163, 149 / 134 / 165; 40: 196 / 155 / 202, 201 / 159 / 206;
+// 180: 581 / 401 / 394, 604 / 406 / 417; and at 0.1 c 128: 446 / 309 / 320, 200: 625 / 443 / 429 (a Harris sheet
+// of 200: 670 / 458 / 439). So 16 lanes from 16 on; 32 from 180, where the two lines cross for cool plasmas (hot: 3 % slower there).
+// Plain, tile push / 32 lanes (16 lanes never better): 24: 222 / 241, 233 / 249; 30: 250 / 255, 261 / 267;
+// 32: 264 / 266, 278 / 276; 34: 284 / 277, 299 / 285; 40: 306 / 294, 323 / 304; 64: 424 / 339, 455 / 358;
+// 128: 744 / 482, 811 / 525; and at 0.1 c 180: 1007 / 625. A Harris sheet on 256x130 cells, two steps and a snapshot: 30:
+// 275 / 270, 32: 285 / 276. So from 30 on: the lines cross at 33 for an even plasma and below 30 for a sheet,
+// whose dense cells hold most of its particles.
 int cells_lanes(const pbpic_handle* h) {
   if (h->cfg.compat != 0 || (!h->mixed && (h->cfg.options & PBPIC_OPT_EXACT_FP64))) return 0;
   const double per_cell = (double)h->n / (double)h->ncells;
