@@ -611,7 +611,8 @@ __global__ void __launch_bounds__(FT) k_field_step(FieldParams<T> a) {
   if (threadIdx.x == 0) *a.ticket = 0;
 }
 
-// Batched domains: grid row blockIdx.y works on domain blockIdx.y.
+// Batched domains: grid row blockIdx.y works on domain blockIdx.y, the phases in launches of their own: a
+// batched step is 13 launches (tests/test_gpu_batch.py counts them), and k_field_step per domain has not been tried in it.
 template <class T>
 __global__ void k_bhalf_batched(const FieldParams<T>* d) {
   __shared__ FieldParams<T> a;

@@ -31,14 +31,14 @@
 // What bounds it, and why this form (512x256 Harris sheet, 26.2 M particles): the tile
 // push of kernels_push.cuh takes 575 us, 14.7 warp instructions a
 // particle at 65 % issue, a third of them moving registers, decoding cells and running
-// the crossers' branch for one or two lanes. This form takes 366 us with
+// the crossers' branch for one or two lanes. This form takes 357 us with
 // 10.0 warp instructions a particle at 72 % issue: bound by instruction issue.
-// On the way there: particles loaded into registers one pass ahead, 540 us and 45 % of
+// On the way there, each with those before it: particles loaded into registers one pass ahead, 540 us and 45 % of
 // the warps' time waiting for loads (the permutation entry, one pass
 // ahead, then the particle: two DRAM latencies in one pass's time); dx, dy, ux, uy as one
 // 16-byte record in place of four arrays, 450 us; the particles by asynchronous
 // copies, 435 us at any depth, because the permutation entries still came one
-// pass ahead; those through the ring too, 370 us. Blocks of 4 warps, 5 per SM at 96
+// pass ahead; those through the ring too, 370 us; the species table and the crossers' one record below, 357 us. Blocks of 4 warps, 5 per SM at 96
 // registers (4 per SM: 385 us; 6 per SM spill: 500 us). A species' constants come from a
 // table in shared memory, with zero charge and mass for lanes beyond the cell, and a
 // crosser is queued as one 16-byte record: 10.7 -> 10.0 instructions, step 453 -> 442 us.

@@ -1569,7 +1569,7 @@ namespace {
 
 constexpr int64_t kStaticKeys = PBPIC_STATIC_SORT_MAX_KEYS;
 constexpr int64_t kStaticHist = RBINS * ((kStaticKeys + RTILE - 1) / RTILE);
-constexpr int64_t kStaticScan = 1024;  // chunk totals of every scan level of the histogram (needs 19)
+constexpr int64_t kStaticScan = 1024;  // chunk totals of every scan level of the histogram (needs 35)
 constexpr int64_t kStaticWords = 4 * kStaticKeys + kStaticHist + kStaticScan + 64;
 
 static __device__ __align__(256) int32_t g_static_sort_scratch[kStaticWords];
@@ -1951,7 +1951,7 @@ int batch_enqueue_step(pbpic_batch* b, int par) {
   CKLAUNCH("k_bhalf_batched");
   k_nodes_batched<float><<<dim3(b->gx_nodes, D), 256, 0, s>>>(b->d_field);
   CKLAUNCH("k_nodes_batched");
-  k_cell_records_batched<<<dim3(grid_for(b->gx_field * 256, 256), D), 256, 0, s>>>(b->d_field);
+  k_cell_records_batched<<<dim3(b->gx_field, D), 256, 0, s>>>(b->d_field);
   CKLAUNCH("k_cell_records_batched");
   k_energy_rows_batched<<<D, 256, 0, s>>>(b->d_erow, ctr + 2);
   CKLAUNCH("k_energy_rows_batched");
